@@ -24,9 +24,7 @@
 // multiplied before dQ(t-1) has released its K), V two.  Warps 0-15 do the element-wise work (thread = TMEM lane,
 // each group of four warps takes 32 of a tile's 128 score columns) in two phases, exponentials then dS; warp 16 is
 // the TMA producer, warp 17 issues all MMAs.  All waits are bounded.
-#include "fa_utils.cuh"
-#include "fa_internal.h"
-#include "sm100_ptx.cuh"
+#include "bwd_sm100_common.cuh"
 #include <atomic>
 
 namespace fa {
@@ -85,22 +83,6 @@ enum { E_FIX = 0, E_RF0, E_RF1, E_RE0, E_RE1, E_S0, E_S1, E_P0, E_P1, E_F0, E_F1
 // barriers of the dQ kernel: KF/KE, VF/VE K and V stage full / free; S scores done; SA scores read; DP dP done; DS dS stored
 enum { G_FIX = 0, G_KF0, G_KF1, G_KF2, G_KE0, G_KE1, G_KE2, G_VF0, G_VF1, G_VE0, G_VE1, G_S0, G_S1, G_SA0, G_SA1, G_DP, G_DS,
        G_ACC, G_COUNT };
-
-// 32 accumulator columns -> the row, scaled and rounded; `left` = columns of the row that remain from dst on (the
-// kernels run a head dim padded to 64 / 128, the row holds the call's own head dim)
-template <typename T>
-__device__ __forceinline__ void store_row_scaled(T* dst, const uint32_t (&r)[32], float s, int left) {
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-        if (v * 8 >= left) break;
-        uint4 pk;
-        pk.x = Elem<T>::pack(__uint_as_float(r[8 * v + 0]) * s, __uint_as_float(r[8 * v + 1]) * s);
-        pk.y = Elem<T>::pack(__uint_as_float(r[8 * v + 2]) * s, __uint_as_float(r[8 * v + 3]) * s);
-        pk.z = Elem<T>::pack(__uint_as_float(r[8 * v + 4]) * s, __uint_as_float(r[8 * v + 5]) * s);
-        pk.w = Elem<T>::pack(__uint_as_float(r[8 * v + 6]) * s, __uint_as_float(r[8 * v + 7]) * s);
-        reinterpret_cast<uint4*>(dst)[v] = pk;
-    }
-}
 
 // ------------------------------------------------------------------------------------------------------
 // dK / dV
@@ -758,7 +740,7 @@ __global__ void __launch_bounds__(192, 1) bwd_dq_from_ds_sm100_kernel(const __gr
             const uint32_t s0 = sbase + st * kStage;
             // A: the dS^T tile as stored ([chunk][key][16 B], no swizzle): 8 keys of a chunk are 128 contiguous bytes,
             // chunks are 2048 bytes apart, a K step of 16 keys is 256 bytes further on; B: the K tile (128-byte swizzle)
-            const uint64_t dA = umma_desc_mn_noswizzle(s0, 128, 2048), dB = umma_desc(s0 + 2 * L::kSub, L::kSub, 1024);
+            const uint64_t dA = umma_desc_noswizzle(s0, 128, 2048), dB = umma_desc(s0 + 2 * L::kSub, L::kSub, 1024);
             umma_ss_group4<0, 16, 32, 48, 0, 128, 256, 384>(tmem, dA, dB, IDESC, j > 0);
             umma_ss_group4<64, 80, 96, 112, 512, 640, 768, 896>(tmem, dA, dB, IDESC, 1);
             umma_commit_w(bar(H_KE0 + st));
@@ -840,6 +822,22 @@ __global__ void __launch_bounds__(256) bwd_delta_sm100_kernel(const fa_bwd_param
     }
 }
 
+template <typename T, int D>
+static void launch_delta_t(const fa_bwd_params& p, float* delta, cudaStream_t st) {
+    const int64_t rows = (p.cu_seqlens_q ? p.total_q : (int64_t)p.b * p.sq) * p.hq;
+    constexpr int kRowsPerBlock = 8 * 1 * (32 / (D / 8));      // warps x rows in flight x rows per warp pass
+    const int64_t want = (rows + kRowsPerBlock - 1) / kRowsPerBlock;
+    const unsigned blocks = (unsigned)(want < 148 * 16 ? (want < 1 ? 1 : want) : 148 * 16);
+    bwd_delta_sm100_kernel<T, D><<<blocks, 256, 0, st>>>(p, delta);
+}
+int launch_bwd_delta_sm100(const fa_bwd_params& p, float* delta) {
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(p.stream);
+    if (p.dtype == FA_F16) p.d <= 64 ? launch_delta_t<__half, 64>(p, delta, st) : p.d <= 128 ? launch_delta_t<__half, 128>(p, delta, st) : launch_delta_t<__half, 256>(p, delta, st);
+    else p.d <= 64 ? launch_delta_t<__nv_bfloat16, 64>(p, delta, st) : p.d <= 128 ? launch_delta_t<__nv_bfloat16, 128>(p, delta, st) : launch_delta_t<__nv_bfloat16, 256>(p, delta, st);
+    mark_kernel(st);
+    return cuda_ok(cudaGetLastError(), "bwd_delta launch");
+}
+
 // 1 (default): dense calls hand dS^T from the dK/dV kernel to a one-GEMM dQ kernel through the workspace;
 // 0: the dQ kernel always recomputes S and dP (fa_debug_set key 7)
 static std::atomic<int> g_ds_spill{1};
@@ -879,15 +877,7 @@ size_t bwd_sm100_workspace(const fa_bwd_params& p) { return delta_bytes(p) + ds_
 
 template <typename T, int D>
 static int launch_bwd_sm100_t(const fa_bwd_params& p, Sm100BwdArgs& a, float* delta, cudaStream_t st) {
-    const int64_t toks = p.cu_seqlens_q ? p.total_q : (int64_t)p.b * p.sq;
-    const int64_t rows = toks * p.hq;
-    {
-        constexpr int kRowsPerBlock = 8 * 1 * (32 / (D / 8));      // warps x rows in flight x rows per warp pass
-        const int64_t want = (rows + kRowsPerBlock - 1) / kRowsPerBlock;
-        const unsigned blocks = (unsigned)(want < 148 * 16 ? (want < 1 ? 1 : want) : 148 * 16);
-        bwd_delta_sm100_kernel<T, D><<<blocks, 256, 0, st>>>(p, delta);
-    }
-    mark_kernel(st);
+    if (int e = launch_bwd_delta_sm100(p, delta)) return e;
     const bool bias = p.softcap > 0.f || p.alibi_slopes;
     auto k1 = bias ? bwd_dkdv_sm100_kernel<T, D, true> : bwd_dkdv_sm100_kernel<T, D, false>;
     auto k2 = bias ? bwd_dq_sm100_kernel<T, D, true> : bwd_dq_sm100_kernel<T, D, false>;

@@ -271,10 +271,11 @@ static int run_backward(const fa_bwd_params& pin) {
     if (p.window_right >= p.sq - 1) p.window_right = -1;
     mark_kernel(reinterpret_cast<cudaStream_t>(p.stream));
     const bool fast = g_policy == 0 && bwd_sm100_supported(p);
-    const size_t need = fast ? bwd_sm100_workspace(p) : bwd_generic_workspace(p);
+    const bool wide = g_policy == 0 && bwd_wide_sm100_supported(p);
+    const size_t need = fast ? bwd_sm100_workspace(p) : wide ? bwd_wide_sm100_workspace(p) : bwd_generic_workspace(p);
     if (!p.workspace || p.workspace_bytes < need)
         return fail(FA_ERR_WORKSPACE, "workspace of %zu bytes required, %zu given", need, p.workspace_bytes);
-    return fast ? launch_bwd_sm100(p) : launch_bwd_generic(p);
+    return fast ? launch_bwd_sm100(p) : wide ? launch_bwd_wide_sm100(p) : launch_bwd_generic(p);
 }
 
 int fa_bwd(const fa_bwd_params* p) {
@@ -293,6 +294,7 @@ int fa_varlen_bwd(const fa_bwd_params* p) {
 
 size_t fa_bwd_workspace_bytes(const fa_bwd_params* p) {
     if (!p || p->hq <= 0) return 0;
+    if (bwd_wide_sm100_supported(*p)) return bwd_wide_sm100_workspace(*p);
     const size_t a = bwd_generic_workspace(*p), b = bwd_sm100_workspace(*p);
     return a > b ? a : b;
 }

@@ -66,6 +66,12 @@ int launch_mla_pair(const fa_mla_params& p, int nsplit, int tokens_per_split, fl
                     int final_direct, cudaStream_t st);
 int mla_pair_error_flag(bool clear);
 int launch_bwd_sm100(const fa_bwd_params& p);
+int launch_bwd_delta_sm100(const fa_bwd_params& p, float* delta);     // delta[token][head] = sum dO o O, head dims up to 256
+// head dims above 128 (bwd_wide_sm100.cu)
+bool bwd_wide_sm100_supported(const fa_bwd_params& p);
+size_t bwd_wide_sm100_workspace(const fa_bwd_params& p);
+int launch_bwd_wide_sm100(const fa_bwd_params& p);
+int bwd_wide_error_flag(bool clear);
 // 1 (default): dense calls hand dS^T tiles from the dK/dV kernel to a one-GEMM dQ kernel (fa_debug_set key 7)
 void bwd_sm100_set_ds_spill(int v);
 // true while the caller has lent per-kernel timing events to this thread

@@ -1068,7 +1068,9 @@ int sm100_error_flag(bool clear) {
     int v = 0;
     cudaMemcpyFromSymbol(&v, g_fwd_sm100_error, sizeof(int));
     if (clear) { int z = 0; cudaMemcpyToSymbol(g_fwd_sm100_error, &z, sizeof(int)); }
-    const int w = bwd_sm100_error_flag(clear);
+    int w = bwd_sm100_error_flag(clear);
+    const int w2 = bwd_wide_error_flag(clear);
+    if (!w) w = w2;
     const int m = mla_pair_error_flag(clear);
     return v ? v : (w ? w : m);
 }

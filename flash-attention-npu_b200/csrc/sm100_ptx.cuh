@@ -215,15 +215,15 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo_bytes
     d |= static_cast<uint64_t>(2) << 61;     // SWIZZLE_128B
     return d;
 }
-// Shared-memory matrix descriptor WITHOUT swizzle for an MN-major operand stored as [chunk of 8 MN elements][k][16 bytes]:
-// eight consecutive k rows of one chunk are a contiguous 128-byte core matrix; `k_group_bytes` = distance between
-// 8-row groups along K (leading offset), `mn_chunk_bytes` = distance between neighbouring 8-element chunks along MN
-// (stride offset).
-__device__ __forceinline__ uint64_t umma_desc_mn_noswizzle(uint32_t saddr, uint32_t k_group_bytes, uint32_t mn_chunk_bytes) {
+// Shared-memory matrix descriptor WITHOUT swizzle: the operand is made of 8 x 16-byte core matrices, each 128 contiguous
+// bytes (eight consecutive rows of 16 bytes).  `k_stride` = distance between neighbouring core matrices along K (leading
+// offset), `mn_stride` = along M or N (stride offset).  Which way a core matrix lies (K-major or MN-major) is the
+// instruction descriptor's business.
+__device__ __forceinline__ uint64_t umma_desc_noswizzle(uint32_t saddr, uint32_t k_stride, uint32_t mn_stride) {
     uint64_t d = 0;
     d |= static_cast<uint64_t>((saddr & 0x3FFFF) >> 4);
-    d |= static_cast<uint64_t>((k_group_bytes >> 4) & 0x3FFF) << 16;
-    d |= static_cast<uint64_t>((mn_chunk_bytes >> 4) & 0x3FFF) << 32;
+    d |= static_cast<uint64_t>((k_stride >> 4) & 0x3FFF) << 16;
+    d |= static_cast<uint64_t>((mn_stride >> 4) & 0x3FFF) << 32;
     d |= static_cast<uint64_t>(1) << 46;     // descriptor version (sm_100)
     return d;
 }

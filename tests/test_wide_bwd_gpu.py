@@ -1,0 +1,94 @@
+"""Backward at head dims above 128 on the tcgen05 kernels: edges of the 128-row tiles, padded head dims, groups, windows,
+packed sequences, several launches; against the float64 oracle, larger shapes against the general kernels."""
+import pytest
+import torch
+
+from oracle import attention_oracle as orc
+from parity import assert_within
+
+pytestmark = pytest.mark.gpu
+
+# (dtype, B, H, Hkv, Sq, Sk, D, causal, wl, wr, softcap)
+CASES = [
+    (torch.bfloat16, 2, 2, 2, 128, 128, 256, False, -1, -1, 0.0),
+    (torch.float16, 1, 4, 2, 129, 127, 192, True, -1, -1, 0.0),
+    (torch.bfloat16, 1, 6, 2, 1, 300, 136, True, -1, -1, 0.0),
+    (torch.float16, 1, 2, 1, 300, 1, 256, False, -1, -1, 0.0),
+    (torch.bfloat16, 1, 2, 2, 700, 513, 248, True, -1, -1, 0.0),
+    (torch.bfloat16, 1, 4, 1, 520, 520, 256, True, 100, 0, 0.0),
+    (torch.float16, 2, 2, 2, 260, 300, 160, False, 40, 70, 0.0),
+    (torch.bfloat16, 1, 2, 1, 300, 300, 200, True, -1, -1, 5.0),
+]
+
+
+def _grads(q, k, v, do, scale, causal, window, cap, slopes=None):
+    import fa_b200_capi as capi
+    from flash_attn_npu import flash_attn_npu as ext
+    out, lse, _, _ = ext.fwd(q, k, v, None, slopes, 0.0, scale, causal, *window, cap, False, None)
+    g = [torch.full_like(t, 777.0) for t in (q, k, v)]
+    ext.bwd(do, q, k, v, out, lse, *g, slopes, 0.0, scale, causal, *window, cap, False, None, None)
+    torch.cuda.synchronize()
+    assert capi.lib.fa_debug_get(2) == 0
+    return g, capi.last_kernel()
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(str(x).replace("torch.", "") for x in c))
+def test_wide_backward_against_the_oracle(case):
+    dt, b, h, hkv, sq, sk, d, causal, wl, wr, cap = case
+    q, do = ((torch.rand(b, sq, h, d) * 2 - 1).to(dt) for _ in range(2))
+    k, v = ((torch.rand(b, sk, hkv, d) * 2 - 1).to(dt) for _ in range(2))
+    scale = d ** -0.5
+    _, lse = orc.attention_fwd(q.float(), k.float(), v.float(), scale, causal, (wl, wr), cap, data_type=torch.float32)
+    lp = orc.attention_bwd(q, k, v, do, lse, scale, causal, (wl, wr), cap)
+    f32 = orc.attention_bwd(q.float(), k.float(), v.float(), do.float(), lse, scale, causal, (wl, wr), cap)
+    got, name = _grads(q.cuda(), k.cuda(), v.cuda(), do.cuda(), scale, causal, (wl, wr), cap)
+    assert name == "sm100_tcgen05_bwd_wide"
+    for n, g, a, r in zip(("dq", "dk", "dv"), got, lp, f32):
+        assert_within(n, g.cpu(), a, r, roundings=3)
+
+
+@pytest.mark.parametrize("d", [192, 256])
+def test_wide_packed_backward_against_the_oracle(d):
+    import fa_b200_capi as capi
+    from flash_attn_npu import flash_attn_npu as ext
+    lq, lk, h, hkv, dt = [300, 0, 129, 64], [260, 70, 400, 1], 4, 2, torch.bfloat16
+    q, do = (torch.randn(sum(lq), h, d).to(dt) for _ in range(2))
+    k, v = (torch.randn(sum(lk), hkv, d).to(dt) for _ in range(2))
+    cu = [torch.tensor([0] + torch.tensor(x).cumsum(0).tolist(), dtype=torch.int32) for x in (lq, lk)]
+    scale = d ** -0.5
+    _, lse32 = orc.attention_varlen_fwd(q.float(), k.float(), v.float(), *cu, scale, True, data_type=torch.float32)
+    lp = orc.attention_varlen_bwd(q, k, v, do, lse32, *cu, scale, True)
+    f32 = orc.attention_varlen_bwd(q.float(), k.float(), v.float(), do.float(), lse32, *cu, scale, True)
+    qg, kg, vg, dog, cq, ck = (t.cuda() for t in (q, k, v, do, *cu))
+    out, lse, _, _ = ext.varlen_fwd(qg, kg, vg, None, cq, ck, None, None, None, None, max(lq), max(lk), 0.0, scale, False, True,
+                                    -1, -1, 0.0, False, None)
+    g = [torch.full_like(t, 777.0) for t in (qg, kg, vg)]
+    ext.varlen_bwd(dog, qg, kg, vg, out, lse, *g, cq, ck, None, max(lq), max(lk), 0.0, scale, False, True, -1, -1, 0.0, False,
+                   None, None)
+    torch.cuda.synchronize()
+    assert capi.last_kernel() == "sm100_tcgen05_bwd_wide" and capi.lib.fa_debug_get(2) == 0
+    for n, x, a, r in zip(("dq", "dk", "dv"), g, lp, f32):
+        assert_within(n, x.cpu(), a, r, roundings=3)
+
+
+@pytest.mark.parametrize("b,sq,sk,h,hkv,causal", [(9, 1024, 1100, 8, 8, True), (2, 2048, 2048, 8, 2, True), (3, 1000, 900, 6, 3, False)])
+def test_wide_backward_over_several_launches(b, sq, sk, h, hkv, causal):
+    """More KV heads than one launch's tiles hold, long walks: against the general kernels.  Both round P, dS and the
+    result to the input type once and sum in fp32, in another order: three half-ulp roundings of the largest value."""
+    import fa_b200_capi as capi
+    dt, d = torch.bfloat16, 256
+    q, do = (torch.randn(b, sq, h, d, device="cuda", dtype=dt) for _ in range(2))
+    k, v = (torch.randn(b, sk, hkv, d, device="cuda", dtype=dt) for _ in range(2))
+    slopes = torch.rand(h, device="cuda") * 0.2
+    got, name = _grads(q, k, v, do, 0.07, causal, (-1, -1), 0.0, slopes)
+    assert name == "sm100_tcgen05_bwd_wide"
+    again, _ = _grads(q, k, v, do, 0.07, causal, (-1, -1), 0.0, slopes)
+    capi.lib.fa_set_kernel_policy(1)
+    try:
+        ref, name = _grads(q, k, v, do, 0.07, causal, (-1, -1), 0.0, slopes)
+        assert name == "generic_mma_bwd"
+    finally:
+        capi.lib.fa_set_kernel_policy(0)
+    for n, x, y, r in zip(("dq", "dk", "dv"), got, again, ref):
+        assert torch.equal(x, y), n
+        assert (x.float() - r.float()).abs().max().item() <= 3 * 2.0 ** -8 * r.float().abs().max().item(), n
