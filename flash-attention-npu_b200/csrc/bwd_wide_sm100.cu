@@ -577,7 +577,7 @@ int launch_bwd_wide_sm100(const fa_bwd_params& p) {
     a.p_tiles = reinterpret_cast<unsigned char*>(p.workspace) + delta_bytes(p);
     a.ds_tiles = a.p_tiles + (size_t)units_per_launch(p) * (unit_bytes(p) / 2);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(p.stream);
-    note_kernel("sm100_tcgen05_bwd_wide");
+    note_kernel("sm100_wide_tcgen05_bwd");
     if (int e = launch_bwd_delta_sm100(p, delta)) return e;
     if (p.dtype == FA_F16) return p.d <= 192 ? launch_t<__half, 192>(p, a, st) : launch_t<__half, 256>(p, a, st);
     return p.d <= 192 ? launch_t<__nv_bfloat16, 192>(p, a, st) : launch_t<__nv_bfloat16, 256>(p, a, st);

@@ -42,7 +42,7 @@ def test_wide_backward_against_the_oracle(case):
     lp = orc.attention_bwd(q, k, v, do, lse, scale, causal, (wl, wr), cap)
     f32 = orc.attention_bwd(q.float(), k.float(), v.float(), do.float(), lse, scale, causal, (wl, wr), cap)
     got, name = _grads(q.cuda(), k.cuda(), v.cuda(), do.cuda(), scale, causal, (wl, wr), cap)
-    assert name == "sm100_tcgen05_bwd_wide"
+    assert name == "sm100_wide_tcgen05_bwd"
     for n, g, a, r in zip(("dq", "dk", "dv"), got, lp, f32):
         assert_within(n, g.cpu(), a, r, roundings=3)
 
@@ -66,7 +66,7 @@ def test_wide_packed_backward_against_the_oracle(d):
     ext.varlen_bwd(dog, qg, kg, vg, out, lse, *g, cq, ck, None, max(lq), max(lk), 0.0, scale, False, True, -1, -1, 0.0, False,
                    None, None)
     torch.cuda.synchronize()
-    assert capi.last_kernel() == "sm100_tcgen05_bwd_wide" and capi.lib.fa_debug_get(2) == 0
+    assert capi.last_kernel() == "sm100_wide_tcgen05_bwd" and capi.lib.fa_debug_get(2) == 0
     for n, x, a, r in zip(("dq", "dk", "dv"), g, lp, f32):
         assert_within(n, x.cpu(), a, r, roundings=3)
 
@@ -81,7 +81,7 @@ def test_wide_backward_over_several_launches(b, sq, sk, h, hkv, causal):
     k, v = (torch.randn(b, sk, hkv, d, device="cuda", dtype=dt) for _ in range(2))
     slopes = torch.rand(h, device="cuda") * 0.2
     got, name = _grads(q, k, v, do, 0.07, causal, (-1, -1), 0.0, slopes)
-    assert name == "sm100_tcgen05_bwd_wide"
+    assert name == "sm100_wide_tcgen05_bwd"
     again, _ = _grads(q, k, v, do, 0.07, causal, (-1, -1), 0.0, slopes)
     capi.lib.fa_set_kernel_policy(1)
     try:
