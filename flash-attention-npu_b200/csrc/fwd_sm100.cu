@@ -5,9 +5,7 @@
 //
 // Every mbarrier wait is bounded; a timeout records a code in g_fwd_sm100_error and the CTA
 // frees its tensor memory and returns.
-#include "fa_utils.cuh"
-#include "fa_internal.h"
-#include "sm100_ptx.cuh"
+#include "fwd_sm100_common.cuh"
 
 namespace fa {
 
@@ -15,39 +13,6 @@ using namespace sm100;
 
 __device__ int g_fwd_sm100_error = 0;
 
-struct alignas(64) Sm100FwdArgs {
-    CUtensorMap tq, tk, tv;
-    void* o;
-    float* lse;
-    int64_t o_sb, o_ss, o_sh;
-    int64_t lse_sb, lse_sh, lse_ss;
-    const int32_t* cu_q;
-    const int32_t* cu_k;
-    // KV-cache calls: device-resident lengths, page table, cache row of a batch entry
-    const int32_t* seqused_k;
-    const int32_t* block_table;
-    const int32_t* cache_batch_idx;
-    int64_t bt_stride;
-    int page_size, s_new;
-    int b, sq, sk, hq, hkv;
-    int d;                               // the call's head dim (a multiple of 8): the kernels run the next of 64 / 128 / 192 / 256, the tile copies
-                                         // zero-fill the columns past d and the epilogue stores d columns
-    float scale_log2;
-    int causal, wl, wr;
-    // score transforms of the BIAS instantiation: softcap (0 = off) and alibi slopes ((hq) or (b,hq), null = off)
-    float softcap, cap_in;               // cap_in = scale / softcap
-    const float* alibi;
-    int64_t alibi_sb;
-    int kv_box;                          // rows of one K/V copy: 128, or 64 when pages are an odd multiple of 64 tokens
-    int gq;                              // two-tile kernel: 1, or the query group size when a KV head's heads are stacked into the tile rows
-    // split-KV (two-tile kernel, cache calls): split s of a sequence takes keys [s * keys_per_split, (s + 1) * ...) and
-    // leaves a normalised fp32 partial output and its LSE for the combine kernel (nsplit = 1: final output directly)
-    int nsplit, keys_per_split;          // keys_per_split is a multiple of 128
-    float* o_part;                       // (nsplit, rows_all, D), rows_all = batch * sq * hq, row = (b * sq + qpos) * hq + head
-    float* lse_part;                     // (nsplit, rows_all)
-    int64_t rows_all;
-    int chunk, nheads_grid;              // grid order, see the kernels: (batch entry, head) pairs a chunk; heads of the grid
-};
 
 // =================================================================================================
 // Two query tiles per CTA (256 rows), P kept in tensor memory.
@@ -1009,6 +974,12 @@ static int sm100_stack_factor(const fa_fwd_params& p) {
     const int G = p.hq / p.hkv;
     return (!p.cu_seqlens_q && p.d <= 128 && p.sq < 128 && G > 1 && G <= 128 && (G & (G - 1)) == 0) ? G : 1;
 }
+// Capped scores without alibi go to the kernel with one query tile a CTA (fwd_single_sm100.cu: the measurements behind
+// this line); alibi, with or without a cap, stays with the BIAS instantiation here.
+static bool single_tile(const fa_fwd_params& p, int gq, int nsplit) {
+    const long blocks = ((long)p.sq * gq + 127) / 128 * nsplit;
+    return p.d <= 128 && p.softcap > 0.f && !p.alibi_slopes && blocks <= 65535;        // a grid dimension
+}
 // CTAs of one split of a dense / cache call
 long fwd_sm100_ctas(const fa_fwd_params& p) {
     const int gq = sm100_stack_factor(p);
@@ -1059,7 +1030,8 @@ int launch_fwd_sm100(const fa_fwd_params& p, int nsplit, int keys_per_split, flo
         if (p.dtype == FA_F16) return p.d <= 192 ? launch_sm100_wide_t<__half, 192>(p, a) : launch_sm100_wide_t<__half, 256>(p, a);
         return p.d <= 192 ? launch_sm100_wide_t<__nv_bfloat16, 192>(p, a) : launch_sm100_wide_t<__nv_bfloat16, 256>(p, a);
     }
-    note_kernel("sm100_tcgen05_2q");
+    note_kernel("sm100_tcgen05_2q");                         // one name for the tcgen05 forward at head dims up to 128
+    if (single_tile(p, a.gq, a.nsplit)) return launch_fwd_single_sm100(p, a);
     if (p.dtype == FA_F16) return p.d <= 64 ? launch_sm100_t<__half, 64>(p, a) : launch_sm100_t<__half, 128>(p, a);
     return p.d <= 64 ? launch_sm100_t<__nv_bfloat16, 64>(p, a) : launch_sm100_t<__nv_bfloat16, 128>(p, a);
 }
@@ -1071,6 +1043,7 @@ int sm100_error_flag(bool clear) {
     int w = bwd_sm100_error_flag(clear);
     const int w2 = bwd_wide_error_flag(clear);
     if (!w) w = w2;
+    if (!w) w = fwd_single_error_flag(clear);
     const int m = mla_pair_error_flag(clear);
     return v ? v : (w ? w : m);
 }

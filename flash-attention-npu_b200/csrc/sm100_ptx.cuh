@@ -353,6 +353,18 @@ __device__ __forceinline__ void umma_ts_group4(uint32_t d_tmem, uint32_t a_tmem,
           "n"(C0), "n"(C0 + CSTEP), "n"(C0 + 2 * CSTEP), "n"(C0 + 3 * CSTEP),
           "n"(B0), "n"(B0 + BSTEP), "n"(B0 + 2 * BSTEP), "n"(B0 + 3 * BSTEP) : "memory");
 }
+// The same with A columns and B offsets listed one by one.
+template <uint32_t C0, uint32_t C1, uint32_t C2, uint32_t C3, uint32_t B0, uint32_t B1, uint32_t B2, uint32_t B3>
+__device__ __forceinline__ void umma_ts_quad(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_base, uint32_t idesc, uint32_t acc0) {
+    asm volatile(
+        "{\n\t.reg .pred q, p0, p1;\n\t.reg .b64 db;\n\t.reg .b32 ta, y;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p0, %5, 0;\n\tsetp.eq.b32 p1, 0, 0;\n\t"
+        FA_UMMA_TS_STEP("%6", "%10", "p0") FA_UMMA_TS_STEP("%7", "%11", "p1") FA_UMMA_TS_STEP("%8", "%12", "p1") FA_UMMA_TS_STEP("%9", "%13", "p1")
+        "}"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(static_cast<uint32_t>(b_base)), "r"(static_cast<uint32_t>(b_base >> 32)), "r"(idesc), "r"(acc0),
+          "n"(C0), "n"(C1), "n"(C2), "n"(C3), "n"(B0), "n"(B1), "n"(B2), "n"(B3) : "memory");
+}
 #undef FA_UMMA_TS_STEP
 // [128 x N] scores = A x B^T over KSTEPS * 16 head dims, both operands K-major tiles of 64-dim sub-tiles SUB bytes apart
 template <int KSTEPS, uint32_t SUB>
