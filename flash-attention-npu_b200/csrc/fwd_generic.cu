@@ -10,6 +10,7 @@
 // scores scaled, soft-capped, masked; online softmax in fp32; P rounded to the input type
 // before P.V while the row sum uses the unrounded P; O = acc / l rounded once;
 // LSE = m + ln l; rows without a visible key give O = 0, LSE = +inf.
+#include <cstring>
 #include "fa_utils.cuh"
 #include "fa_internal.h"
 
@@ -408,13 +409,129 @@ __global__ void append_rotary_kernel(const fa_fwd_params p, T* q_rot, int rotate
         dst[e] = rotate_elem<T>(src, e, rd, p.rotary_interleaved, cosb + (int64_t)pos * (rd / 2), sinb + (int64_t)pos * (rd / 2));
 }
 
+// The same in 16-byte pieces: a thread takes two 8-element chunks of a row, for rotated columns the two that hold each
+// other's partners (non-interleaved: rotary_dim / 2 apart; interleaved: neighbours).  Bound by HBM; the element-wise
+// kernel above, one 64-thread block a row and two bytes a load, took 48 us for the 512 new tokens x 4 sequences of a
+// prefill chunk (32 / 8 heads of 128, 50 MB moved) against 11.6 here.  Same operations in the same order, so the same bits.
+template <typename T>
+__device__ __forceinline__ void rotate_pair8(const uint4 a, const uint4 b, const uint4 cv, const uint4 sv, uint4& oa, uint4& ob) {
+    const T *xa = reinterpret_cast<const T*>(&a), *xb = reinterpret_cast<const T*>(&b);
+    const T *c = reinterpret_cast<const T*>(&cv), *s = reinterpret_cast<const T*>(&sv);
+    T *ya = reinterpret_cast<T*>(&oa), *yb = reinterpret_cast<T*>(&ob);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const float fa_ = Elem<T>::to_float(xa[e]), fb = Elem<T>::to_float(xb[e]), fc = Elem<T>::to_float(c[e]), fs = Elem<T>::to_float(s[e]);
+        ya[e] = Elem<T>::from_float(__fsub_rn(__fmul_rn(fa_, fc), __fmul_rn(fb, fs)));
+        yb[e] = Elem<T>::from_float(__fadd_rn(__fmul_rn(fa_, fs), __fmul_rn(fb, fc)));
+    }
+}
+template <typename T>
+__device__ __forceinline__ uint4 rotate_interleaved8(const uint4 a, const uint2 cv, const uint2 sv) {
+    const T *x = reinterpret_cast<const T*>(&a), *c = reinterpret_cast<const T*>(&cv), *s = reinterpret_cast<const T*>(&sv);
+    uint4 o;
+    T* y = reinterpret_cast<T*>(&o);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float f0 = Elem<T>::to_float(x[2 * e]), f1 = Elem<T>::to_float(x[2 * e + 1]), fc = Elem<T>::to_float(c[e]), fs = Elem<T>::to_float(s[e]);
+        y[2 * e] = Elem<T>::from_float(__fsub_rn(__fmul_rn(f0, fc), __fmul_rn(f1, fs)));
+        y[2 * e + 1] = Elem<T>::from_float(__fadd_rn(__fmul_rn(f0, fs), __fmul_rn(f1, fc)));
+    }
+    return o;
+}
+// unit u of a row of n elements: rotated (rd > 0 and u < rd / 16) or copied; src and dst may be the same address
+template <typename T>
+__device__ __forceinline__ void rotate_unit(T* dst, const T* src, int u, int n, int rd, int interleaved, const T* cosr, const T* sinr) {
+    const uint4* s4 = reinterpret_cast<const uint4*>(src);
+    uint4* d4 = reinterpret_cast<uint4*>(dst);
+    if (u < rd / 16) {
+        if (interleaved) {
+            const uint4 c = *reinterpret_cast<const uint4*>(cosr + u * 8), s = *reinterpret_cast<const uint4*>(sinr + u * 8);
+            const uint4 a = s4[2 * u], b = s4[2 * u + 1];
+            d4[2 * u] = rotate_interleaved8<T>(a, make_uint2(c.x, c.y), make_uint2(s.x, s.y));
+            d4[2 * u + 1] = rotate_interleaved8<T>(b, make_uint2(c.z, c.w), make_uint2(s.z, s.w));
+        } else {
+            uint4 oa, ob;
+            rotate_pair8<T>(s4[u], s4[u + rd / 16], *reinterpret_cast<const uint4*>(cosr + u * 8), *reinterpret_cast<const uint4*>(sinr + u * 8), oa, ob);
+            d4[u] = oa;
+            d4[u + rd / 16] = ob;
+        }
+    } else {                                                 // columns past rotary_dim (a multiple of 16)
+        const bool two = 2 * u + 1 < n / 8;
+        const uint4 a = s4[2 * u];
+        if (two) d4[2 * u + 1] = s4[2 * u + 1];
+        d4[2 * u] = a;
+    }
+}
+template <typename T>
+__global__ void __launch_bounds__(128) append_rotary_vec_kernel(const fa_fwd_params p, T* q_rot, int rotate_q_by_pos, int uk, int uv, int kv_items, int items) {
+    const int item = blockIdx.x * 128 + threadIdx.x;
+    if (item >= items) return;
+    const int b = blockIdx.z;
+    const int L = p.seqused_k[b];
+    const int rd = p.rotary_cos ? p.rotary_dim : 0;
+    const T* cosb = reinterpret_cast<const T*>(p.rotary_cos);
+    const T* sinb = reinterpret_cast<const T*>(p.rotary_sin);
+    if (item < kv_items) {                                   // uk units of the new key row, then uv of the new value row
+        const int row = item / (uk + uv), u = item % (uk + uv);
+        const int i = row / p.hkv, h = row % p.hkv;
+        const int pos = L + i;
+        // a length that points outside the cache (or past the page-table row) appends nothing
+        if (pos < 0 || pos >= p.sk) return;
+        int64_t outer, rin;
+        if (p.block_table) {
+            outer = p.block_table[(int64_t)b * p.block_table_stride + pos / p.page_size];
+            rin = pos % p.page_size;
+        } else {
+            outer = p.cache_batch_idx ? p.cache_batch_idx[b] : b;
+            rin = pos;
+        }
+        if (u < uk) {
+            const int cpos = max(0, min(pos, p.seqlen_ro - 1));
+            const T* src = reinterpret_cast<const T*>(p.k_new.ptr) + (int64_t)b * p.k_new.stride_b + (int64_t)i * p.k_new.stride_s + (int64_t)h * p.k_new.stride_h;
+            T* dst = reinterpret_cast<T*>(p.k.ptr) + outer * p.k.stride_b + rin * p.k.stride_s + (int64_t)h * p.k.stride_h;
+            rotate_unit<T>(dst, src, u, p.d, rd, p.rotary_interleaved, cosb + (int64_t)cpos * (rd / 2), sinb + (int64_t)cpos * (rd / 2));
+        } else {
+            const T* src = reinterpret_cast<const T*>(p.v_new.ptr) + (int64_t)b * p.v_new.stride_b + (int64_t)i * p.v_new.stride_s + (int64_t)h * p.v_new.stride_h;
+            T* dst = reinterpret_cast<T*>(p.v.ptr) + outer * p.v.stride_b + rin * p.v.stride_s + (int64_t)h * p.v.stride_h;
+            rotate_unit<T>(dst, src, u - uk, p.dv, 0, 0, nullptr, nullptr);
+        }
+        return;
+    }
+    const int qi = item - kv_items;
+    const int row = qi / uk, u = qi % uk;
+    const int i = row / p.hq, h = row % p.hq;
+    const int pos = max(0, min(L + (rotate_q_by_pos ? i : 0), p.seqlen_ro - 1));
+    const T* src = reinterpret_cast<const T*>(p.q.ptr) + (int64_t)b * p.q.stride_b + (int64_t)i * p.q.stride_s + (int64_t)h * p.q.stride_h;
+    T* dst = q_rot + (((int64_t)b * p.sq + i) * p.hq + h) * p.d;
+    rotate_unit<T>(dst, src, u, p.d, rd, p.rotary_interleaved, cosb + (int64_t)pos * (rd / 2), sinb + (int64_t)pos * (rd / 2));
+}
+
+// The 16-byte kernel wants 16-byte table rows: rotary_dim a multiple of 16 and aligned tables (the tensors' rows are
+// aligned by the checks at the entry points).  It reads whole chunks before it writes them, so k_new may not be a view
+// of the cache rows it is appended to; nor could it for the element-wise kernel.
+static bool append_rotary_vec_ok(const fa_fwd_params& p, int64_t items) {
+    if (items > (1 << 30) || p.b > 65535) return false;
+    if (!p.rotary_cos) return true;
+    return p.rotary_dim % 16 == 0 && (reinterpret_cast<uintptr_t>(p.rotary_cos) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.rotary_sin) & 15) == 0;
+}
+
 int launch_append_rotary(const fa_fwd_params& p, void* q_rot, int rotate_q_by_pos) {
     const int rows = p.s_new * p.hkv + (q_rot ? p.sq * p.hq : 0);
     if (rows == 0 || p.b == 0) return FA_OK;
-    dim3 grid(rows, 1, p.b);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(p.stream);
-    if (p.dtype == FA_F16) append_rotary_kernel<__half><<<grid, 64, 0, st>>>(p, reinterpret_cast<__half*>(q_rot), rotate_q_by_pos);
-    else append_rotary_kernel<__nv_bfloat16><<<grid, 64, 0, st>>>(p, reinterpret_cast<__nv_bfloat16*>(q_rot), rotate_q_by_pos);
+    const int uk = (p.d + 15) / 16, uv = (p.dv + 15) / 16;
+    const int64_t kv_items = p.k_new.ptr ? (int64_t)p.s_new * p.hkv * (uk + uv) : 0;
+    const int64_t items = kv_items + (q_rot ? (int64_t)p.sq * p.hq * uk : 0);
+    if (items == 0) return FA_OK;
+    if (append_rotary_vec_ok(p, items)) {
+        dim3 grid((unsigned)((items + 127) / 128), 1, p.b);
+        if (p.dtype == FA_F16) append_rotary_vec_kernel<__half><<<grid, 128, 0, st>>>(p, reinterpret_cast<__half*>(q_rot), rotate_q_by_pos, uk, uv, (int)kv_items, (int)items);
+        else append_rotary_vec_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(p, reinterpret_cast<__nv_bfloat16*>(q_rot), rotate_q_by_pos, uk, uv, (int)kv_items, (int)items);
+    } else {
+        dim3 grid(rows, 1, p.b);
+        if (p.dtype == FA_F16) append_rotary_kernel<__half><<<grid, 64, 0, st>>>(p, reinterpret_cast<__half*>(q_rot), rotate_q_by_pos);
+        else append_rotary_kernel<__nv_bfloat16><<<grid, 64, 0, st>>>(p, reinterpret_cast<__nv_bfloat16*>(q_rot), rotate_q_by_pos);
+    }
     mark_kernel(st);
     return cuda_ok(cudaGetLastError(), "append_rotary launch");
 }
@@ -512,6 +629,89 @@ __global__ void __launch_bounds__(kCombineWarps * 32) combine_kernel(
     if (lane == 0 && lse) lse[loff] = (tot > 0.f || keep_minus_inf) ? l : INFINITY;
 }
 
+// The same for few splits: one thread per four columns of a row, all its loads (LSEs and partials) in flight at once, the
+// weights computed by every thread of the row for itself.  Bound by memory latency and bandwidth: the kernel above waits
+// for the LSEs before it asks for a partial, one row a warp; 37 us against this kernel's 22 for the two
+// splits of 65536 rows of 128 (prefill chunk, 80 MB), 6.2 against 3.9 for 8 splits of 128 rows.  Up to 8 splits: beyond that the repeated exponentials cost more than the wait.
+constexpr int kCombineFew = 8;
+template <typename OutT> struct Out4 { using V = float4; };
+template <> struct Out4<__half> { using V = uint2; };
+template <> struct Out4<__nv_bfloat16> { using V = uint2; };
+template <typename OutT, int NS>
+__global__ void __launch_bounds__(256) combine_few_kernel(
+    const float* __restrict__ o_part, const float* __restrict__ lse_part, int64_t o_split_stride, int64_t o_row_stride,
+    int64_t lse_split_stride, OutT* o, float* lse, int nsplit, int64_t rows, int dv,
+    int hq, int sq_dense, int64_t o_sb, int64_t o_ss, int64_t o_sh, int64_t l_sb, int64_t l_sh, int64_t l_ss, int keep_minus_inf) {
+    const int64_t id = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int cols = dv / 4;
+    const int64_t row = id / cols;
+    const int c = (int)(id % cols) * 4;
+    if (row >= rows) return;
+    float ls[NS];
+    float4 v[NS];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) ls[s] = s < nsplit ? __ldg(lse_part + s * lse_split_stride + row) : -INFINITY;
+#pragma unroll
+    for (int s = 0; s < NS; ++s)
+        v[s] = s < nsplit ? __ldg(reinterpret_cast<const float4*>(o_part + row * o_row_stride + s * o_split_stride + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float m = -INFINITY;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) m = fmaxf(m, ls[s]);
+    const float ms = m == -INFINITY ? 0.f : m;
+    float tot = 0.f;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) tot += expf(ls[s] - ms);
+    const float l = tot > 0.f ? ms + logf(tot) : -INFINITY;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        const float w = ls[s] == -INFINITY ? 0.f : expf(ls[s] - l);
+        if (w == 0.f) continue;                              // a split that saw no key: its O slot may hold anything
+        acc.x += w * v[s].x; acc.y += w * v[s].y; acc.z += w * v[s].z; acc.w += w * v[s].w;
+    }
+    const int64_t tok = row / hq;
+    const int head = (int)(row % hq);
+    int64_t ooff, loff;
+    if (sq_dense > 0) {
+        const int64_t bb = tok / sq_dense, qp = tok % sq_dense;
+        ooff = bb * o_sb + qp * o_ss + head * o_sh;
+        loff = bb * l_sb + head * l_sh + qp * l_ss;
+    } else {
+        ooff = tok * o_ss + head * o_sh;
+        loff = head * l_sh + tok * l_ss;
+    }
+    OutT out[4];
+    store_out<OutT>(out, acc.x); store_out<OutT>(out + 1, acc.y); store_out<OutT>(out + 2, acc.z); store_out<OutT>(out + 3, acc.w);
+    typename Out4<OutT>::V pk;
+    memcpy(&pk, out, sizeof(pk));
+    *reinterpret_cast<typename Out4<OutT>::V*>(o + ooff + c) = pk;
+    if (c == 0 && lse) lse[loff] = (tot > 0.f || keep_minus_inf) ? l : INFINITY;
+}
+
+// 16-byte reads of the partials and four outputs a store; several warps may share a row, so the LSEs are not written
+// where they are read
+template <typename OutT>
+static bool combine_few_ok(const float* o_part, const float* lse_part, int64_t lse_split_stride, int64_t rows, const float* lse, int64_t o_split_stride,
+                           int64_t o_row_stride, const OutT* o, int nsplit, int dv, int64_t o_sb, int64_t o_ss, int64_t o_sh) {
+    if (lse && lse >= lse_part && lse < lse_part + (nsplit - 1) * lse_split_stride + rows) return false;
+    return nsplit <= kCombineFew && dv % 4 == 0 && o_split_stride % 4 == 0 && o_row_stride % 4 == 0 && o_sb % 4 == 0 && o_ss % 4 == 0 && o_sh % 4 == 0 &&
+           (reinterpret_cast<uintptr_t>(o_part) & 15) == 0 && (reinterpret_cast<uintptr_t>(o) & (4 * sizeof(OutT) - 1)) == 0;
+}
+template <typename OutT>
+static void launch_combine_kernel(cudaStream_t st, const float* o_part, const float* lse_part, int64_t o_split_stride, int64_t o_row_stride,
+                                  int64_t lse_split_stride, OutT* o, float* lse, int nsplit, int64_t rows, int dv, int hq, int sq_dense,
+                                  int64_t o_sb, int64_t o_ss, int64_t o_sh, int64_t l_sb, int64_t l_sh, int64_t l_ss, int keep) {
+    const int64_t few_blocks = (rows * (dv / 4) + 255) / 256;
+    if (few_blocks > 0 && few_blocks < (1ll << 31) && combine_few_ok<OutT>(o_part, lse_part, lse_split_stride, rows, lse, o_split_stride, o_row_stride, o, nsplit, dv, o_sb, o_ss, o_sh)) {
+        auto k = nsplit <= 2 ? combine_few_kernel<OutT, 2> : nsplit <= 4 ? combine_few_kernel<OutT, 4> : combine_few_kernel<OutT, kCombineFew>;
+        k<<<(unsigned)few_blocks, 256, 0, st>>>(o_part, lse_part, o_split_stride, o_row_stride, lse_split_stride, o, lse, nsplit, rows, dv,
+                                                hq, sq_dense, o_sb, o_ss, o_sh, l_sb, l_sh, l_ss, keep);
+        return;
+    }
+    combine_kernel<OutT><<<(unsigned)((rows + kCombineWarps - 1) / kCombineWarps), kCombineWarps * 32, 0, st>>>(
+        o_part, lse_part, o_split_stride, o_row_stride, lse_split_stride, o, lse, nsplit, rows, dv, hq, sq_dense, o_sb, o_ss, o_sh, l_sb, l_sh, l_ss, keep);
+}
+
 int launch_fwd_combine(const fa_fwd_params& p, int nsplit, const float* o_part, const float* lse_part, int to_partial) {
     // rows are enumerated as (token, head)
     const int64_t toks = p.cu_seqlens_q ? (int64_t)p.total_q : (int64_t)p.b * p.sq;
@@ -519,21 +719,16 @@ int launch_fwd_combine(const fa_fwd_params& p, int nsplit, const float* o_part, 
     if (rows == 0) return FA_OK;
     if (nsplit > kCombineMaxSplits) return fail(FA_ERR_BAD_SHAPE, "at most %d splits can be combined", kCombineMaxSplits);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(p.stream);
-    const int wpb = kCombineWarps;
-    dim3 grid((unsigned)((rows + wpb - 1) / wpb));
     const int sq_dense = p.cu_seqlens_q ? 0 : p.sq;
-    if (to_partial) {
-        combine_kernel<float><<<grid, wpb * 32, 0, st>>>(o_part, lse_part, rows * p.dv, p.dv, rows, p.o_partial, p.lse_partial,
-                                                        nsplit, rows, p.dv, p.hq, 0, 0, (int64_t)p.hq * p.dv, p.dv, 0, 1, p.hq, 1);
-    } else if (p.dtype == FA_F16) {
-        combine_kernel<__half><<<grid, wpb * 32, 0, st>>>(o_part, lse_part, rows * p.dv, p.dv, rows, reinterpret_cast<__half*>(p.o.ptr), p.lse,
-                                                         nsplit, rows, p.dv, p.hq, sq_dense, p.o.stride_b, p.o.stride_s, p.o.stride_h,
-                                                         p.lse_stride_b, p.lse_stride_h, p.lse_stride_s, 0);
-    } else {
-        combine_kernel<__nv_bfloat16><<<grid, wpb * 32, 0, st>>>(o_part, lse_part, rows * p.dv, p.dv, rows, reinterpret_cast<__nv_bfloat16*>(p.o.ptr), p.lse,
-                                                                nsplit, rows, p.dv, p.hq, sq_dense, p.o.stride_b, p.o.stride_s, p.o.stride_h,
-                                                                p.lse_stride_b, p.lse_stride_h, p.lse_stride_s, 0);
-    }
+    if (to_partial)
+        launch_combine_kernel<float>(st, o_part, lse_part, rows * p.dv, p.dv, rows, p.o_partial, p.lse_partial, nsplit, rows, p.dv,
+                                     p.hq, 0, 0, (int64_t)p.hq * p.dv, p.dv, 0, 1, p.hq, 1);
+    else if (p.dtype == FA_F16)
+        launch_combine_kernel<__half>(st, o_part, lse_part, rows * p.dv, p.dv, rows, reinterpret_cast<__half*>(p.o.ptr), p.lse, nsplit, rows, p.dv,
+                                      p.hq, sq_dense, p.o.stride_b, p.o.stride_s, p.o.stride_h, p.lse_stride_b, p.lse_stride_h, p.lse_stride_s, 0);
+    else
+        launch_combine_kernel<__nv_bfloat16>(st, o_part, lse_part, rows * p.dv, p.dv, rows, reinterpret_cast<__nv_bfloat16*>(p.o.ptr), p.lse, nsplit, rows, p.dv,
+                                             p.hq, sq_dense, p.o.stride_b, p.o.stride_s, p.o.stride_h, p.lse_stride_b, p.lse_stride_h, p.lse_stride_s, 0);
     mark_kernel(st);
     return cuda_ok(cudaGetLastError(), "combine launch");
 }
@@ -541,11 +736,8 @@ int launch_fwd_combine(const fa_fwd_params& p, int nsplit, const float* o_part, 
 // public combine entry (flat rows)
 template <typename OutT>
 static void launch_flat_combine(const fa_combine_params& c, cudaStream_t st, int keep = 0) {
-    const int wpb = kCombineWarps;
-    dim3 grid((unsigned)((c.rows + wpb - 1) / wpb));
-    combine_kernel<OutT><<<grid, wpb * 32, 0, st>>>(c.o_partial, c.lse_partial, c.o_split_stride, c.o_row_stride, c.lse_split_stride,
-                                                   reinterpret_cast<OutT*>(c.o), c.lse, c.nsplit, c.rows, c.dv,
-                                                   1, 0, 0, c.o_stride, 0, 0, 0, 1, keep);
+    launch_combine_kernel<OutT>(st, c.o_partial, c.lse_partial, c.o_split_stride, c.o_row_stride, c.lse_split_stride,
+                                reinterpret_cast<OutT*>(c.o), c.lse, c.nsplit, c.rows, c.dv, 1, 0, 0, c.o_stride, 0, 0, 0, 1, keep);
 }
 
 // fp32 output, rows that saw no key keep LSE = -inf (partials that will be combined again)
