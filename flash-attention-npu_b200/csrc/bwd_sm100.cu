@@ -55,9 +55,9 @@ struct alignas(64) Sm100BwdArgs {
                                         // the columns past it, the epilogues store d columns
     float scale, scale_log2;
     int causal, wl, wr;
-    // dS^T tiles handed from the dK/dV kernel to the dQ kernel through global memory (dense calls within the
-    // workspace limit): tile (batch, head, key block n, query block m) = 128 keys x 128 queries of the input type,
-    // stored as [16 chunks of 8 queries][128 keys][8 queries]
+    // dS^T tiles handed from the dK/dV kernel to the dQ kernel through global memory (calls within the workspace limit):
+    // tile (query block, head, key block n of the sequence) = 128 keys x 128 queries of the input type, stored as
+    // [16 chunks of 8 queries][128 keys][8 queries]; see ds_query_block for the numbering of the query blocks
     void* ds_tiles;
     int nkb, nqb;
     // score transforms of the BIAS instantiation of the dK/dV kernel: softcap (0 = off) and alibi slopes (null = off)
@@ -65,6 +65,14 @@ struct alignas(64) Sm100BwdArgs {
     const float* alibi;
     int64_t alibi_sb;
 };
+
+// First query block of sequence b in the numbering of the dS^T tiles.  Packed: the number of query blocks of the sequences
+// before b is only known on the device as a sum; cu_q[b] / 128 + b is at least that and grows by at least the number of
+// blocks of each sequence (ceil(len / 128) <= floor((off + len) / 128) - floor(off / 128) + 1), so blocks never share a
+// number and all numbers lie below total_q / 128 + batch.
+__device__ __forceinline__ int64_t ds_query_block(const Sm100BwdArgs& a, int b, int q_off) {
+    return a.cu_q ? (int64_t)q_off / 128 + b : (int64_t)b * a.nqb;
+}
 
 template <int D>
 struct BwdSm100Smem {
@@ -355,7 +363,7 @@ __global__ void __launch_bounds__(608, 1) bwd_dkdv_sm100_kernel(const __grid_con
             if (a.ds_tiles) {
                 // the same rounded dS^T goes to global memory for the dQ kernel, which then needs one GEMM a tile
                 // instead of recomputing S and dP.  Issued after the hand-off so that the stores are off the chain.
-                const int64_t tile = (((int64_t)b * a.hq + (hk * G + s / nmb)) * a.nkb + bi.x) * a.nqb + (mb_lo + s % nmb);
+                const int64_t tile = ((ds_query_block(a, b, q_off) + mb_lo + s % nmb) * a.hq + (hk * G + s / nmb)) * a.nkb + bi.x;
                 // tile layout [16 chunks of 8 queries][128 keys][16 bytes]: a warp's 32 rows of one chunk are 512
                 // contiguous bytes (one fully coalesced store instruction), and the tile is at the same time the
                 // unswizzled operand layout the dQ kernel's MMA reads
@@ -641,18 +649,28 @@ __global__ void __launch_bounds__(608, 1) bwd_dq_sm100_kernel(const __grid_const
 // ------------------------------------------------------------------------------------------------------
 // dQ from stored dS^T tiles: dQ = scale * sum over key blocks of dS K, one GEMM a tile.  The dK/dV kernel has
 // written every (key block, query block) tile it visited; this kernel visits exactly the same pairs (it derives its
-// key blocks from the dK/dV kernel's rule), streams dS^T and K tiles through a three-stage TMA ring and multiplies.
-// No element-wise work, no exponentials: HBM-bound on reading the dS^T tiles once.
-//   warp 0 TMA producer, warp 1 MMA issuer (also owns the tensor memory), warps 2-5 epilogue (thread = query row)
+// key blocks from the dK/dV kernel's rule), streams dS^T and K tiles through a TMA ring and multiplies.  No element-wise
+// work, no exponentials: bound by reading the dS^T tiles once from HBM and K from L2.  A CTA takes NB query blocks of one
+// head, so that a K tile feeds NB tiles of dS^T: with one block a CTA the two streams together came to what the SMs can
+// read from L2 (10 TB/s over the GPU).
+//   warp 0 TMA producer, warp 1 MMA issuer (also owns the tensor memory), then four epilogue warps a block (thread =
+//   query row)
 // ------------------------------------------------------------------------------------------------------
 enum { H_KF0 = 0, H_KF1, H_KF2, H_KE0, H_KE1, H_KE2, H_ACC, H_COUNT };
+template <int D, int NB>
+struct BwdDqSmem {
+    static constexpr int kDs = 2 * BwdSm100Smem<D>::kSub;                // a dS^T tile
+    static constexpr int kStage = NB * kDs + BwdSm100Smem<D>::kTileB;    // NB dS^T tiles and a K tile
+    static constexpr int kStages = NB == 1 ? 3 : 2;
+    static constexpr int kBytes = kStages * kStage + 256;
+};
 
-template <typename T, int D>
-__global__ void __launch_bounds__(192, 1) bwd_dq_from_ds_sm100_kernel(const __grid_constant__ Sm100BwdArgs a) {
+template <typename T, int D, int NB>
+__global__ void __launch_bounds__(64 + 128 * NB, 1) bwd_dq_from_ds_sm100_kernel(const __grid_constant__ Sm100BwdArgs a) {
     using L = BwdSm100Smem<D>;
+    using H = BwdDqSmem<D, NB>;
     constexpr int NSUB = D / 64;
-    constexpr int kStage = 2 * L::kSub + L::kTileB;          // dS^T tile (128 x 128) + K tile (128 x D)
-    constexpr uint32_t TMEM_COLS = D <= 64 ? 64 : 128;
+    constexpr uint32_t TMEM_COLS = D * NB;
     constexpr int FMT = Elem<T>::kDtype == FA_BF16 ? 1 : 0;
     // M = 128 queries, N = D, K = keys; both operands are read "across" their tiles: A = dS^T tile [key][query]
     // (query-contiguous), B = K tile [key][dim] (dim-contiguous)
@@ -661,44 +679,58 @@ __global__ void __launch_bounds__(192, 1) bwd_dq_from_ds_sm100_kernel(const __gr
     extern __shared__ unsigned char smem_raw[];
     const uint32_t sbase = (smem_addr(smem_raw) + 1023u) & ~1023u;
     unsigned char* sgen = smem_raw + (sbase - smem_addr(smem_raw));
-    const uint32_t bars = sbase + 3 * kStage;
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(sgen + 3 * kStage + 8 * H_COUNT);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sgen + 3 * kStage + 8 * H_COUNT + 8);
+    const uint32_t bars = sbase + H::kStages * H::kStage;
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(sgen + H::kStages * H::kStage + 8 * H_COUNT);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sgen + H::kStages * H::kStage + 8 * H_COUNT + 8);
     auto bar = [&](int i) { return bars + 8u * i; };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int pair = blockIdx.z * a.chunk_q + blockIdx.x;    // grid order as in the dK/dV kernel, over (batch entry, head) pairs
     if (pair >= a.b * a.hq) return;
     const int b = pair / a.hq, h = pair % a.hq;
-    const int mblk = gridDim.y - 1 - blockIdx.y;
-    const int sq = a.sq, sk = a.sk;
-    const int m0 = mblk * 128;
-    if (m0 >= sq) return;
+    const int mb0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * NB;          // first query block
+    int q_off = 0, k_off = 0, sq = a.sq, sk = a.sk;
+    if (a.cu_q) { q_off = a.cu_q[b]; sq = a.cu_q[b + 1] - q_off; k_off = a.cu_k[b]; sk = a.cu_k[b + 1] - k_off; }
+    if (mb0 * 128 >= sq) return;
     if (g_bwd_sm100_error) return;
     const int hk = h / (a.hq / a.hkv);
     const int wl = a.wl, wr = a.causal ? 0 : a.wr;
     const int diff = sk - sq;
-    const int rows = min(128, sq - m0);
-    // key blocks whose dK/dV CTA walked this query block (the rule of bwd_dkdv_sm100_kernel); they form one range
-    int t_lo = a.nkb, t_hi = 0;
-    for (int n = 0; n < a.nkb; ++n) {
-        const int n0 = n * 128, krows = min(128, sk - n0);
-        int i_lo = 0, i_hi = sq - 1;
-        if (wr >= 0) i_lo = max(0, n0 - diff - wr);
-        if (wl >= 0) i_hi = min(sq - 1, n0 + krows - 1 + wl - diff);
-        const int mb_lo = i_lo / 128, mb_hi = i_hi >= i_lo ? i_hi / 128 + 1 : mb_lo;
-        if (mblk >= mb_lo && mblk < mb_hi) { t_lo = min(t_lo, n); t_hi = max(t_hi, n + 1); }
-    }
-    const int ntiles = max(0, t_hi - t_lo);
-    T* dqb = reinterpret_cast<T*>(a.dq) + (int64_t)b * a.dq_sb + (int64_t)m0 * a.dq_ss + (int64_t)h * a.dq_sh;
-    if (ntiles == 0) {
-        if (tid < rows) {
-            const uint4 z = make_uint4(0, 0, 0, 0);
-            T* row = dqb + (int64_t)tid * a.dq_ss;
+    const int nkb = sk > 0 ? min(a.nkb, (sk + 127) / 128) : 0;
+    // key blocks whose dK/dV CTA walked query block mb0 + x (the rule of bwd_dkdv_sm100_kernel); they form one range, empty
+    // for blocks past the end
+    int t_lo[NB], t_hi[NB];
 #pragma unroll
-            for (int c = 0; c < D / 8; ++c)
-                if (c * 8 < a.d) reinterpret_cast<uint4*>(row)[c] = z;      // the call's head dim, not the kernel's padded one
+    for (int x = 0; x < NB; ++x) {
+        int lo = nkb, hi = 0;
+        const int mblk = mb0 + x;
+        for (int n = lane; n < nkb && mblk * 128 < sq; n += 32) {
+            const int n0 = n * 128, krows = min(128, sk - n0);
+            int i_lo = 0, i_hi = sq - 1;
+            if (wr >= 0) i_lo = max(0, n0 - diff - wr);
+            if (wl >= 0) i_hi = min(sq - 1, n0 + krows - 1 + wl - diff);
+            const int mb_lo = i_lo / 128, mb_hi = i_hi >= i_lo ? i_hi / 128 + 1 : mb_lo;
+            if (mblk >= mb_lo && mblk < mb_hi) { lo = min(lo, n); hi = max(hi, n + 1); }
         }
+        t_lo[x] = __reduce_min_sync(0xffffffffu, lo);
+        t_hi[x] = __reduce_max_sync(0xffffffffu, hi);
+    }
+    int u_lo = t_lo[0], u_hi = t_hi[0];                      // key blocks of any of the query blocks
+#pragma unroll
+    for (int x = 1; x < NB; ++x) { u_lo = min(u_lo, t_lo[x]); u_hi = max(u_hi, t_hi[x]); }
+    const int ntiles = max(0, u_hi - u_lo);
+    // rows of query block mb0 + x, row r of it
+    auto dq_row = [&](int x, int r) {
+        return reinterpret_cast<T*>(a.dq) + (a.cu_q ? 0 : (int64_t)b * a.dq_sb) + (int64_t)(q_off + (mb0 + x) * 128 + r) * a.dq_ss + (int64_t)h * a.dq_sh;
+    };
+    auto zero_row = [&](T* row) {
+        const uint4 z = make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int c = 0; c < D / 8; ++c)
+            if (c * 8 < a.d) reinterpret_cast<uint4*>(row)[c] = z;          // the call's head dim, not the kernel's padded one
+    };
+    if (ntiles == 0) {
+        for (int r = tid; r < min(128 * NB, sq - mb0 * 128); r += 64 + 128 * NB) zero_row(dq_row(r / 128, r % 128));
         return;
     }
     if (tid == 0) {
@@ -716,49 +748,69 @@ __global__ void __launch_bounds__(192, 1) bwd_dq_from_ds_sm100_kernel(const __gr
     if (warp == 0) {
         if (lane == 0) {
             tma_prefetch_desc(&a.tk);
+            const int64_t tile0 = ((ds_query_block(a, b, q_off) + mb0) * a.hq + h) * a.nkb;
             bool ok = true;
             for (int j = 0; j < ntiles && ok; ++j) {
-                const int st = j % 3;
-                if (j >= 3) ok = mbar_wait(bar(H_KE0 + st), (j / 3 - 1) & 1, abort_flag, err, 51);
+                const int st = j % H::kStages;
+                if (j >= H::kStages) ok = mbar_wait(bar(H_KE0 + st), (j / H::kStages - 1) & 1, abort_flag, err, 51);
                 if (!ok) break;
-                const int n = t_lo + j;
-                const int64_t tile = (((int64_t)b * a.hq + h) * a.nkb + n) * a.nqb + mblk;
-                mbar_expect_tx(bar(H_KF0 + st), kStage);
-                const uint32_t s0 = sbase + st * kStage;
-                bulk_load_1d(s0, reinterpret_cast<const unsigned char*>(a.ds_tiles) + tile * (128 * 128 * 2), 2 * L::kSub, bar(H_KF0 + st));
+                const int n = u_lo + j;
+                uint32_t bytes = L::kTileB;
 #pragma unroll
-                for (int c = 0; c < NSUB; ++c) tma_load_4d(s0 + 2 * L::kSub + c * L::kSub, &a.tk, bar(H_KF0 + st), c * 64, hk, n * 128, b);
+                for (int x = 0; x < NB; ++x) if (n >= t_lo[x] && n < t_hi[x]) bytes += H::kDs;
+                mbar_expect_tx(bar(H_KF0 + st), bytes);
+                const uint32_t s0 = sbase + st * H::kStage;
+#pragma unroll
+                for (int x = 0; x < NB; ++x)
+                    if (n >= t_lo[x] && n < t_hi[x])
+                        bulk_load_1d(s0 + x * H::kDs, reinterpret_cast<const unsigned char*>(a.ds_tiles) + (tile0 + (int64_t)x * a.hq * a.nkb + n) * H::kDs, H::kDs, bar(H_KF0 + st));
+#pragma unroll
+                for (int c = 0; c < NSUB; ++c) tma_load_4d(s0 + NB * H::kDs + c * L::kSub, &a.tk, bar(H_KF0 + st), c * 64, hk, k_off + n * 128, a.cu_q ? 0 : b);
             }
         }
     } else if (warp == 1) {
         bool ok = true;
         for (int j = 0; j < ntiles && ok; ++j) {
-            const int st = j % 3;
-            ok = mbar_wait(bar(H_KF0 + st), (j / 3) & 1, abort_flag, err, 52);
+            const int st = j % H::kStages, n = u_lo + j;
+            ok = mbar_wait(bar(H_KF0 + st), (j / H::kStages) & 1, abort_flag, err, 52);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t s0 = sbase + st * kStage;
+            const uint32_t s0 = sbase + st * H::kStage;
             // A: the dS^T tile as stored ([chunk][key][16 B], no swizzle): 8 keys of a chunk are 128 contiguous bytes,
             // chunks are 2048 bytes apart, a K step of 16 keys is 256 bytes further on; B: the K tile (128-byte swizzle)
-            const uint64_t dA = umma_desc_noswizzle(s0, 128, 2048), dB = umma_desc(s0 + 2 * L::kSub, L::kSub, 1024);
-            umma_ss_group4<0, 16, 32, 48, 0, 128, 256, 384>(tmem, dA, dB, IDESC, j > 0);
-            umma_ss_group4<64, 80, 96, 112, 512, 640, 768, 896>(tmem, dA, dB, IDESC, 1);
+            const uint64_t dB = umma_desc(s0 + NB * H::kDs, L::kSub, 1024);
+#pragma unroll
+            for (int x = 0; x < NB; ++x) {
+                if (n < t_lo[x] || n >= t_hi[x]) continue;
+                const uint64_t dA = umma_desc_noswizzle(s0 + x * H::kDs, 128, 2048);
+                umma_ss_group4<0, 16, 32, 48, 0, 128, 256, 384>(tmem + x * D, dA, dB, IDESC, n > t_lo[x]);
+                umma_ss_group4<64, 80, 96, 112, 512, 640, 768, 896>(tmem + x * D, dA, dB, IDESC, 1);
+            }
             umma_commit_w(bar(H_KE0 + st));
         }
         if (ok) umma_commit_w(bar(H_ACC));
     } else {
         // Rows of tiles past the last key hold zeros (their probabilities are zero), so nothing needs masking here.
-        const int r = (warp & 3) * 32 + lane;               // warps 2..5 cover the four lane quarters 2,3,0,1
+        const int r = (warp & 3) * 32 + lane;               // warps 2..5, 6..9 cover the four lane quarters 2,3,0,1
+        const int x = (warp - 2) >> 2;
+        const int rows = min(128, sq - (mb0 + x) * 128);     // none for a block past the end
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+        bool any = false;
+#pragma unroll
+        for (int y = 0; y < NB; ++y) if (y == x) any = t_hi[y] > t_lo[y];
         if (mbar_wait(bar(H_ACC), 0, abort_flag, err, 53)) {
             tc_fence_after();
-            T* row = dqb + (int64_t)r * a.dq_ss;
+            T* row = dq_row(x, r);
+            if (any) {
 #pragma unroll
-            for (int c = 0; c < D / 32; ++c) {
-                uint32_t acc[32];
-                tmem_ld32(tmem + lane_base + c * 32, acc);
-                tmem_wait_ld();
-                if (r < rows) store_row_scaled<T>(row + c * 32, acc, a.scale, a.d - c * 32);
+                for (int c = 0; c < D / 32; ++c) {
+                    uint32_t acc[32];
+                    tmem_ld32(tmem + x * D + lane_base + c * 32, acc);
+                    tmem_wait_ld();
+                    if (r < rows) store_row_scaled<T>(row + c * 32, acc, a.scale, a.d - c * 32);
+                }
+            } else if (r < rows) {
+                zero_row(row);
             }
         }
     }
@@ -862,18 +914,23 @@ bool bwd_sm100_supported(const fa_bwd_params& p) {
 }
 
 // The dK/dV kernel can hand its dS^T tiles to the dQ kernel through the workspace (then the backward executes the
-// algorithm's five GEMMs a tile pair instead of seven): dense calls whose tiles fit into this many bytes.
+// algorithm's five GEMMs a tile pair instead of seven): calls whose tiles fit into this many bytes.  For packed calls the
+// host knows only the longest lengths, so the bound counts every query block against the longest key length; what is
+// touched are the tiles of each sequence.
 constexpr size_t kDsTileBytes = 128 * 128 * 2;
 constexpr size_t kDsWorkspaceLimit = (size_t)6 << 30;
 static size_t ds_tiles_bytes(const fa_bwd_params& p) {
-    if (p.cu_seqlens_q || p.cu_seqlens_k || p.b <= 0) return 0;
-    const size_t tiles = (size_t)p.b * p.hq * ((p.sk + 127) / 128) * ((p.sq + 127) / 128);
-    const size_t bytes = tiles * kDsTileBytes;
+    if (p.b <= 0) return 0;
+    const size_t nqb = p.cu_seqlens_q ? (size_t)p.total_q / 128 + p.b : (size_t)p.b * ((p.sq + 127) / 128);
+    const size_t bytes = nqb * p.hq * ((p.sk + 127) / 128) * kDsTileBytes;
     return bytes <= kDsWorkspaceLimit ? bytes : 0;
 }
 static size_t delta_bytes(const fa_bwd_params& p) { return (bwd_generic_workspace(p) + 255) & ~(size_t)255; }
 
 size_t bwd_sm100_workspace(const fa_bwd_params& p) { return delta_bytes(p) + ds_tiles_bytes(p); }
+size_t bwd_sm100_workspace_min(const fa_bwd_params& p) { return delta_bytes(p); }
+
+constexpr int kDqPairMin = 8;                                // query blocks an SM from which a CTA takes two
 
 template <typename T, int D>
 static int launch_bwd_sm100_t(const fa_bwd_params& p, Sm100BwdArgs& a, float* delta, cudaStream_t st) {
@@ -885,15 +942,20 @@ static int launch_bwd_sm100_t(const fa_bwd_params& p, Sm100BwdArgs& a, float* de
     if (int e = cuda_ok(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute")) return e;
     if (a.ds_tiles) {
         // five-GEMM path: the dQ kernel consumes the dS^T tiles the dK/dV kernel leaves, so it runs after it
-        auto k3 = bwd_dq_from_ds_sm100_kernel<T, D>;
-        const int smem3 = 3 * (2 * BwdSm100Smem<D>::kSub + BwdSm100Smem<D>::kTileB) + 256 + 1024;
-        if (int e = cuda_ok(cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, smem3), "cudaFuncSetAttribute")) return e;
+        // Two query blocks a CTA in dense calls once that leaves every SM several CTAs: the whole training step at B4 S4096
+        // H32 D128 causal 2243 -> 2217 us.  Below that, and for packed sequences with their uneven lengths (B12 of 128-4096
+        // tokens, H16/4: 1159 us with one block, 1176 with two), the shorter CTAs fill the GPU better.
         const unsigned nk = (unsigned)((p.sk + 127) / 128), nq = (unsigned)((p.sq + 127) / 128);
+        const unsigned zq = (unsigned)(((int64_t)p.b * p.hq + a.chunk_q - 1) / a.chunk_q);
+        const int nb = !p.cu_seqlens_q && (int64_t)p.b * p.hq * nq >= (int64_t)kDqPairMin * sm_count() ? 2 : 1;
+        auto k3 = nb == 2 ? bwd_dq_from_ds_sm100_kernel<T, D, 2> : bwd_dq_from_ds_sm100_kernel<T, D, 1>;
+        const int smem3 = (nb == 2 ? BwdDqSmem<D, 2>::kBytes : BwdDqSmem<D, 1>::kBytes) + 1024;
+        if (int e = cuda_ok(cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, smem3), "cudaFuncSetAttribute")) return e;
         dim3 g1(a.chunk_kv, nk, (unsigned)(((int64_t)p.b * p.hkv + a.chunk_kv - 1) / a.chunk_kv));
-        dim3 g3(a.chunk_q, nq, (unsigned)(((int64_t)p.b * p.hq + a.chunk_q - 1) / a.chunk_q));
+        dim3 g3(a.chunk_q, (nq + nb - 1) / nb, zq);
         k1<<<g1, 608, smem, st>>>(a);
         mark_kernel(st);
-        k3<<<g3, 192, smem3, st>>>(a);
+        k3<<<g3, 64 + 128 * nb, smem3, st>>>(a);
         mark_kernel(st);
         return cuda_ok(cudaGetLastError(), "bwd_sm100 launch");
     }
@@ -902,8 +964,8 @@ static int launch_bwd_sm100_t(const fa_bwd_params& p, Sm100BwdArgs& a, float* de
     const unsigned nk = (unsigned)((p.sk + 127) / 128), nq = (unsigned)((p.sq + 127) / 128);
     dim3 g1(a.chunk_kv, nk, (unsigned)(((int64_t)p.b * p.hkv + a.chunk_kv - 1) / a.chunk_kv));
     dim3 g2(a.chunk_q, nq, (unsigned)(((int64_t)p.b * p.hq + a.chunk_q - 1) / a.chunk_q));
-    // packed calls and calls beyond the workspace limit: the dQ kernel recomputes S and dP; both kernels on the
-    // caller's stream, one after the other
+    // calls beyond the workspace limit: the dQ kernel recomputes S and dP; both kernels on the caller's stream, one after
+    // the other
     k1<<<g1, 608, smem, st>>>(a);
     mark_kernel(st);
     k2<<<g2, 608, smem_dq, st>>>(a);
@@ -942,7 +1004,7 @@ int launch_bwd_sm100(const fa_bwd_params& p) {
     a.causal = p.causal; a.wl = p.window_left; a.wr = p.window_right;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(p.stream);
     float* delta = reinterpret_cast<float*>(p.workspace);
-    note_kernel(a.ds_tiles ? "sm100_tcgen05_bwd_5gemm" : "sm100_tcgen05_bwd");
+    note_kernel(a.ds_tiles && !packed ? "sm100_tcgen05_bwd_5gemm" : "sm100_tcgen05_bwd");     // the packed call keeps one name
     if (p.dtype == FA_F16) return p.d <= 64 ? launch_bwd_sm100_t<__half, 64>(p, a, delta, st) : launch_bwd_sm100_t<__half, 128>(p, a, delta, st);
     return p.d <= 64 ? launch_bwd_sm100_t<__nv_bfloat16, 64>(p, a, delta, st) : launch_bwd_sm100_t<__nv_bfloat16, 128>(p, a, delta, st);
 }

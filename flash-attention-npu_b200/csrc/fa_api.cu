@@ -272,7 +272,7 @@ static int run_backward(const fa_bwd_params& pin) {
     mark_kernel(reinterpret_cast<cudaStream_t>(p.stream));
     const bool fast = g_policy == 0 && bwd_sm100_supported(p);
     const bool wide = g_policy == 0 && bwd_wide_sm100_supported(p);
-    const size_t need = fast ? bwd_sm100_workspace(p) : wide ? bwd_wide_sm100_workspace(p) : bwd_generic_workspace(p);
+    const size_t need = fast ? bwd_sm100_workspace_min(p) : wide ? bwd_wide_sm100_workspace(p) : bwd_generic_workspace(p);
     if (!p.workspace || p.workspace_bytes < need)
         return fail(FA_ERR_WORKSPACE, "workspace of %zu bytes required, %zu given", need, p.workspace_bytes);
     return fast ? launch_bwd_sm100(p) : wide ? launch_bwd_wide_sm100(p) : launch_bwd_generic(p);
@@ -292,12 +292,14 @@ int fa_varlen_bwd(const fa_bwd_params* p) {
     return run_backward(*p);
 }
 
-size_t fa_bwd_workspace_bytes(const fa_bwd_params* p) {
+static size_t bwd_workspace(const fa_bwd_params* p, size_t (*fast)(const fa_bwd_params&)) {
     if (!p || p->hq <= 0) return 0;
     if (bwd_wide_sm100_supported(*p)) return bwd_wide_sm100_workspace(*p);
-    const size_t a = bwd_generic_workspace(*p), b = bwd_sm100_workspace(*p);
+    const size_t a = bwd_generic_workspace(*p), b = fast(*p);
     return a > b ? a : b;
 }
+size_t fa_bwd_workspace_bytes(const fa_bwd_params* p) { return bwd_workspace(p, bwd_sm100_workspace); }
+size_t fa_bwd_workspace_min_bytes(const fa_bwd_params* p) { return bwd_workspace(p, bwd_sm100_workspace_min); }
 
 int fa_combine(const fa_combine_params* c) {
     if (!c) return fail(FA_ERR_NULL, "params is null");

@@ -79,5 +79,6 @@ bool kernel_events_active();
 bool bwd_sm100_supported(const fa_bwd_params& p);
 size_t bwd_generic_workspace(const fa_bwd_params& p);
 size_t bwd_sm100_workspace(const fa_bwd_params& p);
+size_t bwd_sm100_workspace_min(const fa_bwd_params& p);               // without the dS tiles
 
 }  // namespace fa

@@ -116,6 +116,7 @@ EXPORTS = {
     "fa_bwd": (C.c_int, [C.POINTER(BwdParams)]),
     "fa_varlen_bwd": (C.c_int, [C.POINTER(BwdParams)]),
     "fa_bwd_workspace_bytes": (C.c_size_t, [C.POINTER(BwdParams)]),
+    "fa_bwd_workspace_min_bytes": (C.c_size_t, [C.POINTER(BwdParams)]),
     "fa_combine": (C.c_int, [C.POINTER(CombineParams)]),
     "fa_mla_decode": (C.c_int, [C.POINTER(MlaParams)]),
     "fa_peer_combine": (C.c_int, [C.POINTER(PeerCombineParams)]),

@@ -338,7 +338,10 @@ def _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p
     p.dtype = _dtype_code(q)
     p.deterministic = int(deterministic)
     keep = _alibi(p, alibi_slopes_, batch, hq)
-    ws = capi.workspace(lib.fa_bwd_workspace_bytes(p), q.device)
+    try:
+        ws = capi.workspace(lib.fa_bwd_workspace_bytes(p), q.device)
+    except torch.OutOfMemoryError:                           # without room for the dS tiles the kernels recompute them
+        ws = capi.workspace(lib.fa_bwd_workspace_min_bytes(p), q.device)
     p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
     p.stream = capi.stream_ptr(q.device)
     with torch.cuda.device(q.device):
