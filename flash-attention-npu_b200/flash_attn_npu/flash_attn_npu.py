@@ -13,8 +13,9 @@ from typing import List, Optional
 import torch
 import torch.nn.functional as F
 
+import ctypes
+
 import fa_b200_capi as capi
-from fa_b200_capi import FwdParams, BwdParams, tensor4, ptr, check, lib
 
 
 def _dtype_code(t):
@@ -36,15 +37,33 @@ def _common_checks(q, k, v, softcap, what="key"):
         raise RuntimeError("softcap must be non-negative (0.0 disables softcap)")
 
 
-def _alibi(p, alibi_slopes, batch, nheads):
+def _alibi(alibi_slopes, batch, nheads):
+    """-> (tensor to keep alive, pointer, batch stride)"""
     if alibi_slopes is None:
-        return None
+        return None, 0, 0
     a = alibi_slopes.to(torch.float32).contiguous()
     if a.shape not in ((nheads,), (batch, nheads)):
         raise RuntimeError("alibi_slopes must have shape (nheads,) or (batch_size, nheads)")
-    p.alibi_slopes = a.data_ptr()
-    p.alibi_stride_b = 0 if a.dim() == 1 else a.stride(0)
-    return a
+    return a, a.data_ptr(), 0 if a.dim() == 1 else a.stride(0)
+
+
+def _leaves(t, packed=False):
+    """The four leaves of an fa_tensor: (B,S,H,D), or packed (T,H,D) without a batch stride."""
+    s = t.stride()
+    if s[-1] != 1:
+        raise RuntimeError("last dimension must be contiguous")
+    return (t.data_ptr(), 0, s[0], s[1]) if packed else (t.data_ptr(), s[0], s[1], s[2])
+
+
+_NO_TENSOR = (0, 0, 0, 0)
+
+
+def _ptr(t):
+    return 0 if t is None else t.data_ptr()
+
+
+def _i32(x):
+    return x if -2 ** 31 <= x < 2 ** 31 else ctypes.c_int32(x).value
 
 
 def _pad8(t):
@@ -56,6 +75,18 @@ def fwd(q, k, v, out_, alibi_slopes_, p_dropout, softmax_scale, is_causal, windo
         window_size_right, softcap, return_softmax, gen_) -> List[torch.Tensor]:
     """mha_fwd (flash_api.cpp:639-846). q (B,Sq,H,D), k/v (B,Sk,Hkv,D) ->
     [out, softmax_lse (B,H,Sq) fp32, p (empty), rng_state (int64[2])]."""
+    out, lse = dense_forward(q, k, v, out_, alibi_slopes_, p_dropout, softmax_scale, is_causal, window_size_left,
+                             window_size_right, softcap, return_softmax)
+    return [out, lse, *_unused(q)]
+
+
+def _unused(q):
+    return (torch.empty((0,), dtype=q.dtype, device=q.device), torch.zeros((2,), dtype=torch.int64, device=q.device))
+
+
+def dense_forward(q, k, v, out_, alibi_slopes_, p_dropout, softmax_scale, is_causal, window_size_left,
+                  window_size_right, softcap, return_softmax):
+    """fwd without the two results that carry nothing here (dropout mask and generator state)."""
     _common_checks(q, k, v, softcap)
     if p_dropout != 0.0:
         raise RuntimeError("FlashAttention on B200 does not support dropout.")
@@ -71,30 +102,27 @@ def fwd(q, k, v, out_, alibi_slopes_, p_dropout, softmax_scale, is_causal, windo
         raise RuntimeError("Number of heads in key/value must divide number of heads in query")
     q, k, v = _pad8(q), _pad8(k), _pad8(v)
     d = q.size(-1)
+    device = q.device
     out = torch.empty_like(q) if (out_ is None or d != d_og) else out_
-    lse = torch.empty((batch, hq, sq), dtype=torch.float32, device=q.device)
-    p = FwdParams()
-    p.q, p.k, p.v, p.o = tensor4(q), tensor4(k), tensor4(v), tensor4(out)
-    p.lse = lse.data_ptr()
-    p.lse_stride_b, p.lse_stride_h, p.lse_stride_s = lse.stride(0), lse.stride(1), lse.stride(2)
-    p.b, p.sq, p.sk, p.hq, p.hkv, p.d, p.dv = batch, sq, sk, hq, hkv, d, v.size(-1)
-    p.scale, p.softcap = softmax_scale, softcap
-    p.causal, p.window_left, p.window_right = int(is_causal), window_size_left, window_size_right
-    p.dtype = _dtype_code(q)
-    p.num_splits = 1
-    keep = _alibi(p, alibi_slopes_, batch, hq)
-    p.stream = capi.stream_ptr(q.device)
-    with torch.cuda.device(q.device):
-        check(lib.fa_fwd(p))
+    lse = torch.empty((batch, hq, sq), dtype=torch.float32, device=device)
+    keep, alibi, alibi_sb = _alibi(alibi_slopes_, batch, hq)
+    buf = capi.FWD_BLOCK.new(
+        *_leaves(q), *_leaves(k), *_leaves(v), *_leaves(out), lse.data_ptr(), *lse.stride(),
+        0, 0, 0,                                             # cu_seqlens_q, cu_seqlens_k, seqused_k
+        0, 0, 0, 0, alibi, alibi_sb,                         # block_table, its stride, page_size, cache_batch_idx
+        batch, sq, sk, 0, 0, hq, hkv, d, v.size(-1), softmax_scale, softcap,
+        int(is_causal), _i32(window_size_left), _i32(window_size_right), _dtype_code(q),
+        *_NO_TENSOR, *_NO_TENSOR, 0, 0, 0, 0, 0, 0,          # new keys and values, rotary
+        1, 0, 0, 0, 0, 0, 0, 0, 0, 0,                        # num_splits .. kv_entries
+        capi.raw_stream(device))
+    capi.launch(capi._call_fwd, buf, device)
     del keep
     if d != d_og:
         out = out[..., :d_og]
         if out_ is not None:
             out_.copy_(out)
             out = out_
-    empty_p = torch.empty((0,), dtype=q.dtype, device=q.device)
-    rng_state = torch.zeros((2,), dtype=torch.int64, device=q.device)
-    return [out, lse, empty_p, rng_state]
+    return out, lse
 
 
 def varlen_fwd(q, k, v, out_, cu_seqlens_q, cu_seqlens_k, seqused_k_, leftpad_k_, block_table_,
@@ -102,6 +130,16 @@ def varlen_fwd(q, k, v, out_, cu_seqlens_q, cu_seqlens_k, seqused_k_, leftpad_k_
                is_causal, window_size_left, window_size_right, softcap, return_softmax, gen_):
     """mha_varlen_fwd (flash_api.cpp:848-1089). q (Tq,H,D), k/v (Tk,Hkv,D) or a paged cache
     (blocks,page,Hkv,D) with block_table -> [out, softmax_lse (H,Tq), p, rng_state]."""
+    out, lse = packed_forward(q, k, v, out_, cu_seqlens_q, cu_seqlens_k, seqused_k_, leftpad_k_, block_table_, alibi_slopes_,
+                              max_seqlen_q, max_seqlen_k, p_dropout, softmax_scale, zero_tensors, is_causal,
+                              window_size_left, window_size_right, softcap, return_softmax)
+    return [out, lse, *_unused(q)]
+
+
+def packed_forward(q, k, v, out_, cu_seqlens_q, cu_seqlens_k, seqused_k_, leftpad_k_, block_table_, alibi_slopes_,
+                   max_seqlen_q, max_seqlen_k, p_dropout, softmax_scale, zero_tensors, is_causal, window_size_left,
+                   window_size_right, softcap, return_softmax):
+    """varlen_fwd without the two results that carry nothing here."""
     _common_checks(q, k, v, softcap)
     if p_dropout != 0.0:
         raise RuntimeError("FlashAttention on B200 does not support dropout.")
@@ -124,45 +162,35 @@ def varlen_fwd(q, k, v, out_, cu_seqlens_q, cu_seqlens_k, seqused_k_, leftpad_k_
     out = torch.empty_like(q) if (out_ is None or d != d_og) else out_
     if zero_tensors:
         out.zero_()
-    lse = torch.full((hq, total_q), float("inf"), dtype=torch.float32, device=q.device)
-    p = FwdParams()
-    p.q, p.o = tensor4(q, packed=True), tensor4(out, packed=True)
+    device = q.device
+    lse = torch.full((hq, total_q), float("inf"), dtype=torch.float32, device=device)
+    table = (0, 0, 0)
     if paged:
-        p.k, p.v = tensor4(k), tensor4(v)
         if block_table_.dtype != torch.int32 or block_table_.stride(-1) != 1:
             raise RuntimeError("block_table must be int32 with contiguous last dimension")
-        p.block_table, p.block_table_stride, p.page_size = block_table_.data_ptr(), block_table_.stride(0), k.shape[1]
-        p.kv_entries = min(k.shape[0], v.shape[0])
-        p.seqused_k = ptr(seqused_k_)
-        p.num_splits = 0
-    else:
-        p.k, p.v = tensor4(k, packed=True), tensor4(v, packed=True)
-        p.seqused_k = None
-        p.num_splits = 1
-    p.lse = lse.data_ptr()
-    p.lse_stride_b, p.lse_stride_h, p.lse_stride_s = 0, lse.stride(0), lse.stride(1)
-    p.cu_seqlens_q, p.cu_seqlens_k = cu_seqlens_q.data_ptr(), ptr(cu_seqlens_k)
-    p.b, p.sq, p.sk, p.total_q = batch, max_seqlen_q, max_seqlen_k, total_q
-    p.total_k = 0 if paged else k.shape[0]
-    p.hq, p.hkv, p.d, p.dv = hq, hkv, d, v.size(-1)
-    p.scale, p.softcap = softmax_scale, softcap
-    p.causal, p.window_left, p.window_right = int(is_causal), window_size_left, window_size_right
-    p.dtype = _dtype_code(q)
-    keep = _alibi(p, alibi_slopes_, batch, hq)
-    ws = capi.workspace(lib.fa_fwd_workspace_bytes(p), q.device)
-    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
-    p.stream = capi.stream_ptr(q.device)
-    with torch.cuda.device(q.device):
-        check(lib.fa_varlen_fwd(p))
+        table = (block_table_.data_ptr(), block_table_.stride(0), k.shape[1])
+    keep, alibi, alibi_sb = _alibi(alibi_slopes_, batch, hq)
+    lse_sh, lse_ss = lse.stride()
+    buf = capi.FWD_BLOCK.new(
+        *_leaves(q, True), *_leaves(k, not paged), *_leaves(v, not paged), *_leaves(out, True), lse.data_ptr(), 0, lse_sh, lse_ss,
+        cu_seqlens_q.data_ptr(), _ptr(cu_seqlens_k), _ptr(seqused_k_) if paged else 0, *table, 0, alibi, alibi_sb,
+        batch, max_seqlen_q, max_seqlen_k, total_q, 0 if paged else k.shape[0], hq, hkv, d, v.size(-1), softmax_scale, softcap,
+        int(is_causal), _i32(window_size_left), _i32(window_size_right), _dtype_code(q),
+        *_NO_TENSOR, *_NO_TENSOR, 0, 0, 0, 0, 0, 0,
+        0 if paged else 1, 0, 0, 0, 0, 0, 0, 0, 0, min(k.shape[0], v.shape[0]) if paged else 0,
+        capi.raw_stream(device))
+    nbytes = capi._fwd_bytes(buf)
+    if nbytes:
+        ws = capi.workspace(nbytes, device)
+        capi.set_workspace(capi.FWD_BLOCK, buf, ws, nbytes)
+    capi.launch(capi._call_varlen_fwd, buf, device)
     del keep
     if d != d_og:
         out = out[..., :d_og]
         if out_ is not None:
             out_.copy_(out)
             out = out_
-    empty_p = torch.empty((0,), dtype=q.dtype, device=q.device)
-    rng_state = torch.zeros((2,), dtype=torch.int64, device=q.device)
-    return [out, lse, empty_p, rng_state]
+    return out, lse
 
 
 def kvcache_forward(q, kcache, vcache, k_, v_, seqlens_k_, rotary_cos_, rotary_sin_, cache_batch_idx_,
@@ -201,21 +229,15 @@ def kvcache_forward(q, kcache, vcache, k_, v_, seqlens_k_, rotary_cos_, rotary_s
             raise RuntimeError("appending k/v needs a head dimension that is a multiple of 8")
         q, kcache, vcache = _pad8(q), _pad8(kcache), _pad8(vcache)
     d = q.size(-1)
+    device = q.device
     out = torch.empty_like(q) if (out_ is None or d != d_og) else out_
-    p = FwdParams()
     if packed_q:
-        lse = torch.full((hq, total_q), float("inf"), dtype=torch.float32, device=q.device)
-        p.q, p.o = tensor4(q, packed=True), tensor4(out, packed=True)
-        p.lse_stride_b, p.lse_stride_h, p.lse_stride_s = 0, lse.stride(0), lse.stride(1)
-        p.cu_seqlens_q, p.total_q = cu_seqlens_q.data_ptr(), total_q
+        lse = torch.full((hq, total_q), float("inf"), dtype=torch.float32, device=device)
+        lse_strides = (0, *lse.stride())
     else:
-        lse = torch.empty((batch, hq, sq), dtype=torch.float32, device=q.device)
-        p.q, p.o = tensor4(q), tensor4(out)
-        p.lse_stride_b, p.lse_stride_h, p.lse_stride_s = lse.stride(0), lse.stride(1), lse.stride(2)
-    p.lse = lse.data_ptr()
-    p.k, p.v = tensor4(kcache), tensor4(vcache)
-    p.kv_entries = min(kcache.shape[0], vcache.shape[0])
-    s_new = 0
+        lse = torch.empty((batch, hq, sq), dtype=torch.float32, device=device)
+        lse_strides = lse.stride()
+    new_kv, s_new = _NO_TENSOR + _NO_TENSOR, 0
     if k_ is not None:
         if v_ is None:
             raise RuntimeError("k and v must be passed together")
@@ -223,47 +245,40 @@ def kvcache_forward(q, kcache, vcache, k_, v_, seqlens_k_, rotary_cos_, rotary_s
             raise RuntimeError("seqlens_k must be passed when appending k and v")
         if k_.dtype != q.dtype or v_.dtype != q.dtype:
             raise RuntimeError("new k/v must have the query's dtype")
-        p.k_new, p.v_new = tensor4(k_), tensor4(v_)
-        s_new = k_.shape[1]
-    p.s_new = s_new
+        new_kv, s_new = _leaves(k_) + _leaves(v_), k_.shape[1]
     if paged:
-        p.block_table, p.block_table_stride, p.page_size = block_table_.data_ptr(), block_table_.stride(0), kcache.shape[1]
+        table = (block_table_.data_ptr(), block_table_.stride(0), kcache.shape[1])
         sk = block_table_.shape[1] * kcache.shape[1]
     else:
-        sk = kcache.shape[1]
-    p.seqused_k = ptr(seqlens_k_)
-    p.cache_batch_idx = ptr(cache_batch_idx_)
+        table, sk = (0, 0, 0), kcache.shape[1]
+    rotary = (0, 0, 0, 0, 0)
     if rotary_cos_ is not None:
         if k_ is None:
             raise RuntimeError("rotary embedding is only applied when k and v are passed in")
         rc = rotary_cos_.to(q.dtype).contiguous()
         rs = rotary_sin_.to(q.dtype).contiguous()
-        p.rotary_cos, p.rotary_sin = rc.data_ptr(), rs.data_ptr()
-        p.rotary_dim, p.seqlen_ro = rc.shape[1] * 2, rc.shape[0]
-        p.rotary_interleaved = int(is_rotary_interleaved)
-    p.b, p.sq, p.sk, p.hq, p.hkv, p.d, p.dv = batch, sq, sk, hq, hkv, d, vcache.size(-1)
-    p.scale, p.softcap = softmax_scale, softcap
-    p.causal, p.window_left, p.window_right = int(is_causal), window_size_left, window_size_right
-    p.dtype = _dtype_code(q)
-    p.num_splits = num_splits
-    if kv_range is not None:
-        p.kv_begin, p.kv_end = int(kv_range[0]), int(kv_range[1])
-    if partials is not None:
-        p.partials_only = 1
-        p.o_partial, p.lse_partial = partials[0].data_ptr(), partials[1].data_ptr()
+        rotary = (rc.data_ptr(), rs.data_ptr(), rc.shape[1] * 2, int(is_rotary_interleaved), rc.shape[0])
+    kv_begin, kv_end = (0, 0) if kv_range is None else (int(kv_range[0]), int(kv_range[1]))
+    part = (0, 0, 0) if partials is None else (1, partials[0].data_ptr(), partials[1].data_ptr())
     if sched_meta is not None:
         capi.require_cuda(sched_meta)
         if sched_meta.dtype not in (torch.uint8, torch.int32) or not sched_meta.is_contiguous():
             raise RuntimeError("scheduler_metadata must be the contiguous uint8 / int32 tensor get_scheduler_metadata returned")
-        if sched_meta.numel() * sched_meta.element_size() < 4 * lib.fa_scheduler_metadata_ints(batch) or sched_meta.data_ptr() % 4:
+        if sched_meta.numel() * sched_meta.element_size() < 4 * capi.lib.fa_scheduler_metadata_ints(batch) or sched_meta.data_ptr() % 4:
             raise RuntimeError("scheduler_metadata is too small for this batch size")
-        p.sched_meta = sched_meta.data_ptr()
-    keep = _alibi(p, alibi_slopes_, batch, hq)
-    ws = capi.workspace(lib.fa_fwd_workspace_bytes(p), q.device)
-    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
-    p.stream = capi.stream_ptr(q.device)
-    with torch.cuda.device(q.device):
-        check(lib.fa_fwd_kvcache(p))
+    keep, alibi, alibi_sb = _alibi(alibi_slopes_, batch, hq)
+    buf = capi.FWD_BLOCK.new(
+        *_leaves(q, packed_q), *_leaves(kcache), *_leaves(vcache), *_leaves(out, packed_q), lse.data_ptr(), *lse_strides,
+        cu_seqlens_q.data_ptr() if packed_q else 0, 0, _ptr(seqlens_k_), *table, _ptr(cache_batch_idx_), alibi, alibi_sb,
+        batch, sq, sk, total_q, 0, hq, hkv, d, vcache.size(-1), softmax_scale, softcap,
+        int(is_causal), _i32(window_size_left), _i32(window_size_right), _dtype_code(q),
+        *new_kv, s_new, *rotary, num_splits, kv_begin, kv_end, *part, 0, 0, _ptr(sched_meta),
+        min(kcache.shape[0], vcache.shape[0]), capi.raw_stream(device))
+    nbytes = capi._fwd_bytes(buf)
+    if nbytes:
+        ws = capi.workspace(nbytes, device)
+        capi.set_workspace(capi.FWD_BLOCK, buf, ws, nbytes)
+    capi.launch(capi._call_kvcache, buf, device)
     del keep
     if d != d_og:
         out = out[..., :d_og]
@@ -289,6 +304,7 @@ def fwd_kvcache(q, kcache, vcache, k_, v_, seqlens_k_, rotary_cos_, rotary_sin_,
 
 def _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p_dropout, softmax_scale,
                 is_causal, wl, wr, softcap, deterministic, cu_q=None, cu_k=None, max_sq=0, max_sk=0):
+    """The three gradients."""
     capi.require_cuda(dout, q, k, v, out, softmax_lse)
     if softcap < 0.0:
         raise RuntimeError("softcap must be non-negative (0.0 disables softcap)")
@@ -298,15 +314,16 @@ def _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p
     d_og = q.size(-1)
     if d_og % 8 != 0:
         raise RuntimeError("backward needs a head dimension that is a multiple of 8 (the Python API pads it)")
+    device = q.device
     dq = torch.empty_like(q) if dq_ is None else dq_
     dk = torch.empty_like(k) if dk_ is None else dk_
     dv = torch.empty_like(v) if dv_ is None else dv_
-    p = BwdParams()
-    names = ("dout", "q", "k", "v", "o", "dq", "dk", "dv")
-    for name, t in zip(names, (dout, q, k, v, out, dq, dk, dv)):
-        if t.stride(-1) != 1:
+    leaves = []
+    for t in (dout, q, k, v, out, dq, dk, dv):
+        s = t.stride()
+        if s[-1] != 1:
             raise RuntimeError("Input tensor must have contiguous last dimension")
-        setattr(p, name, tensor4(t, packed=packed))
+        leaves += (t.data_ptr(), 0, s[0], s[1]) if packed else (t.data_ptr(), s[0], s[1], s[2])
     if packed:
         total_q, hq, _ = q.shape
         total_k, hkv, _ = k.shape
@@ -314,53 +331,51 @@ def _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p
             raise RuntimeError("mha_varlen_bwd: softmax_lse for TND must be a 2D tensor.")
         if softmax_lse.shape != (hq, total_q):
             raise RuntimeError("mha_varlen_bwd: softmax_lse must have shape (nheads, total_q)")
-        batch = cu_q.numel() - 1
-        p.cu_seqlens_q, p.cu_seqlens_k = cu_q.data_ptr(), cu_k.data_ptr()
-        p.b, p.sq, p.sk, p.total_q, p.total_k = batch, max_sq, max_sk, total_q, total_k
-        p.lse_stride_b, p.lse_stride_h, p.lse_stride_s = 0, softmax_lse.stride(0), softmax_lse.stride(1)
-        softmax_d = torch.empty((hq, total_q + 128 * batch), dtype=torch.float32, device=q.device)
+        batch, sq, sk = cu_q.numel() - 1, max_sq, max_sk
+        lse_strides = (0, *softmax_lse.stride())
+        cu = (cu_q.data_ptr(), cu_k.data_ptr())
     else:
         batch, sq, hq, _ = q.shape
         sk, hkv = k.shape[1], k.shape[2]
         if softmax_lse.shape != (batch, hq, sq):
             raise RuntimeError("softmax_lse must have shape (batch, nheads, seqlen_q)")
-        p.b, p.sq, p.sk = batch, sq, sk
-        p.lse_stride_b, p.lse_stride_h, p.lse_stride_s = softmax_lse.stride(0), softmax_lse.stride(1), softmax_lse.stride(2)
-        softmax_d = torch.empty((batch, hq, (sq + 127) // 128 * 128), dtype=torch.float32, device=q.device)
+        total_q = total_k = 0
+        lse_strides = softmax_lse.stride()
+        cu = (0, 0)
     if softmax_lse.dtype != torch.float32:
         raise RuntimeError("softmax_lse must be fp32")
     if hq % hkv != 0:
         raise RuntimeError("Number of heads in key/value must divide number of heads in query")
-    p.lse = softmax_lse.data_ptr()
-    p.hq, p.hkv, p.d, p.dv_dim = hq, hkv, q.size(-1), v.size(-1)
-    p.scale, p.softcap = softmax_scale, softcap
-    p.causal, p.window_left, p.window_right = int(is_causal), wl, wr
-    p.dtype = _dtype_code(q)
-    p.deterministic = int(deterministic)
-    keep = _alibi(p, alibi_slopes_, batch, hq)
+    keep, alibi, alibi_sb = _alibi(alibi_slopes_, batch, hq)
+    buf = capi.BWD_BLOCK.new(
+        *leaves, softmax_lse.data_ptr(), *lse_strides, *cu, batch, sq, sk, total_q, total_k, hq, hkv, q.size(-1), v.size(-1),
+        softmax_scale, softcap, int(is_causal), _i32(wl), _i32(wr), _dtype_code(q), int(deterministic), 0, 0,
+        capi.raw_stream(device), alibi, alibi_sb)
     try:
-        ws = capi.workspace(lib.fa_bwd_workspace_bytes(p), q.device)
+        ws = capi.workspace(capi._bwd_bytes(buf), device)
     except torch.OutOfMemoryError:                           # without room for the dS tiles the kernels recompute them
-        ws = capi.workspace(lib.fa_bwd_workspace_min_bytes(p), q.device)
-    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
-    p.stream = capi.stream_ptr(q.device)
-    with torch.cuda.device(q.device):
-        check(lib.fa_varlen_bwd(p) if packed else lib.fa_bwd(p))
-    return [dq, dk, dv, softmax_d]
+        ws = capi.workspace(capi._bwd_min_bytes(buf), device)
+    capi.set_workspace(capi.BWD_BLOCK, buf, ws, ws.numel())
+    capi.launch(capi._call_varlen_bwd if packed else capi._call_bwd, buf, device)
+    del keep
+    return dq, dk, dv
 
 
 def bwd(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p_dropout, softmax_scale, is_causal,
         window_size_left, window_size_right, softcap, deterministic, gen_, rng_state):
     """mha_bwd (flash_api.cpp:1279-1328) -> [dq, dk, dv, softmax_d]."""
-    return _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p_dropout, softmax_scale,
-                       is_causal, window_size_left, window_size_right, softcap, deterministic)
+    dq, dk, dv = _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p_dropout, softmax_scale,
+                             is_causal, window_size_left, window_size_right, softcap, deterministic)
+    batch, sq, hq, _ = q.shape
+    return [dq, dk, dv, torch.empty((batch, hq, (sq + 127) // 128 * 128), dtype=torch.float32, device=q.device)]
 
 
 def varlen_bwd(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, cu_seqlens_q, cu_seqlens_k, alibi_slopes_,
                max_seqlen_q, max_seqlen_k, p_dropout, softmax_scale, zero_tensors, is_causal,
                window_size_left, window_size_right, softcap, deterministic, gen_, rng_state):
     """mha_varlen_bwd (flash_api.cpp:1092-1277) -> [dq, dk, dv, softmax_d]."""
-    res = _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p_dropout, softmax_scale,
-                      is_causal, window_size_left, window_size_right, softcap, deterministic,
-                      cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k)
-    return res
+    dq, dk, dv = _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p_dropout, softmax_scale,
+                             is_causal, window_size_left, window_size_right, softcap, deterministic,
+                             cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k)
+    total_q, hq, _ = q.shape
+    return [dq, dk, dv, torch.empty((hq, total_q + 128 * (cu_seqlens_q.numel() - 1)), dtype=torch.float32, device=q.device)]

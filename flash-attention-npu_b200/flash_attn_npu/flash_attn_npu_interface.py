@@ -10,9 +10,12 @@ from typing import Optional, Tuple, Union
 import torch
 import torch.nn.functional as F
 
+from fa_b200_capi import plain as _plain
 from . import flash_attn_npu as _ext
 
-_BWD_ALIGN = 64   # the backward pads the head dim to a multiple of 64 (reference :23-44)
+# The backward kernels take any multiple of 8 (tile copies fill up to their own 64 / 128 / 192 / 256 columns); the reference
+# pads to 64 (:23-44), which costs five copies of the inputs at head dim 96.
+_BWD_ALIGN = 8
 
 
 def maybe_contiguous(x):
@@ -160,15 +163,28 @@ _wrapped_flash_attn_varlen_backward = _flash_attn_varlen_backward
 # ------------------------------------------------------------------------------------------
 # autograd
 # ------------------------------------------------------------------------------------------
+# Dispatching a custom op from Python costs about as much as the kernels of a small training step (B5 S1024 H4: 70 us of
+# kernels in a call of 275).  Where the dispatch would do nothing but call the body (fa_b200_capi.plain) and the scalars have
+# exactly the schema's types, so that nothing would be converted or refused, the body is called directly.
+def _scalars_ok(dropout_p, softmax_scale, causal, window_size, softcap):
+    return (type(dropout_p) is float and dropout_p == 0.0 and type(softmax_scale) is float and type(causal) is bool
+            and type(window_size[0]) is int and type(window_size[1]) is int and type(softcap) is float)
+
+
 def _dense_forward(ctx, q, k, v, dropout_p, softmax_scale, causal, window_size, softcap, alibi_slopes,
                    deterministic, return_softmax, is_grad):
     if softmax_scale is None:
         softmax_scale = q.shape[-1] ** (-0.5)
     q, k, v, og = _pad_fwd_headdim(q, k, v)
-    out_padded, lse, s_dmask, rng = _wrapped_flash_attn_forward(
-        q, k, v, dropout_p, softmax_scale, causal=causal, window_size_left=window_size[0],
-        window_size_right=window_size[1], softcap=softcap, alibi_slopes=alibi_slopes,
-        return_softmax=return_softmax and dropout_p > 0)
+    if _scalars_ok(dropout_p, softmax_scale, causal, window_size, softcap) and _plain(q, k, v, alibi_slopes):
+        out_padded, lse = _ext.dense_forward(maybe_contiguous(q), maybe_contiguous(k), maybe_contiguous(v), None, alibi_slopes,
+                                             dropout_p, softmax_scale, causal, window_size[0], window_size[1], softcap, False)
+        s_dmask, rng = torch.empty((0,), dtype=q.dtype, device=q.device) if return_softmax else None, None
+    else:
+        out_padded, lse, s_dmask, rng = _wrapped_flash_attn_forward(
+            q, k, v, dropout_p, softmax_scale, causal=causal, window_size_left=window_size[0],
+            window_size_right=window_size[1], softcap=softcap, alibi_slopes=alibi_slopes,
+            return_softmax=return_softmax and dropout_p > 0)
     if is_grad:
         ctx.save_for_backward(q, k, v, out_padded, lse, rng)
         ctx.dropout_p, ctx.softmax_scale, ctx.causal = dropout_p, softmax_scale, causal
@@ -184,9 +200,15 @@ def _dense_backward(ctx, dout, dq=None, dk=None, dv=None):
         views = None
     else:
         views = True
-    _wrapped_flash_attn_backward(dout, q, k, v, out, lse, dq, dk, dv, ctx.dropout_p, ctx.softmax_scale, ctx.causal,
-                                 ctx.window_size[0], ctx.window_size[1], ctx.softcap, ctx.alibi_slopes,
-                                 ctx.deterministic, rng_state=rng)
+    if (_scalars_ok(ctx.dropout_p, ctx.softmax_scale, ctx.causal, ctx.window_size, ctx.softcap) and type(ctx.deterministic) is bool
+            and _plain(dout, q, k, v, out, lse, dq, dk, dv, ctx.alibi_slopes)):
+        _ext._bwd_common(maybe_contiguous(dout), maybe_contiguous(q), maybe_contiguous(k), maybe_contiguous(v), maybe_contiguous(out),
+                         lse, dq, dk, dv, ctx.alibi_slopes, ctx.dropout_p, ctx.softmax_scale, ctx.causal, ctx.window_size[0],
+                         ctx.window_size[1], ctx.softcap, ctx.deterministic)
+    else:
+        _wrapped_flash_attn_backward(dout, q, k, v, out, lse, dq, dk, dv, ctx.dropout_p, ctx.softmax_scale, ctx.causal,
+                                     ctx.window_size[0], ctx.window_size[1], ctx.softcap, ctx.alibi_slopes,
+                                     ctx.deterministic, rng_state=rng)
     return dq[..., :og], dk[..., :og], dv[..., :og], views
 
 
@@ -195,10 +217,17 @@ def _varlen_forward(ctx, q, k, v, cu_q, cu_k, max_q, max_k, dropout_p, softmax_s
     if softmax_scale is None:
         softmax_scale = q.shape[-1] ** (-0.5)
     q, k, v, og = _pad_fwd_headdim(q, k, v)
-    out_padded, lse, s_dmask, rng = _wrapped_flash_attn_varlen_forward(
-        q, k, v, cu_q, cu_k, max_q, max_k, dropout_p, softmax_scale, causal=causal,
-        window_size_left=window_size[0], window_size_right=window_size[1], softcap=softcap,
-        alibi_slopes=alibi_slopes, return_softmax=return_softmax and dropout_p > 0, block_table=block_table)
+    if (_scalars_ok(dropout_p, softmax_scale, causal, window_size, softcap) and type(max_q) is int and type(max_k) is int
+            and isinstance(cu_q, torch.Tensor) and isinstance(cu_k, torch.Tensor) and _plain(q, k, v, cu_q, cu_k, alibi_slopes, block_table)):
+        out_padded, lse = _ext.packed_forward(maybe_contiguous(q), maybe_contiguous(k), maybe_contiguous(v), None, cu_q, cu_k, None, None,
+                                              block_table, alibi_slopes, max_q, max_k, dropout_p, softmax_scale, False, causal,
+                                              window_size[0], window_size[1], softcap, False)
+        s_dmask, rng = torch.empty((0,), dtype=q.dtype, device=q.device) if return_softmax else None, None
+    else:
+        out_padded, lse, s_dmask, rng = _wrapped_flash_attn_varlen_forward(
+            q, k, v, cu_q, cu_k, max_q, max_k, dropout_p, softmax_scale, causal=causal,
+            window_size_left=window_size[0], window_size_right=window_size[1], softcap=softcap,
+            alibi_slopes=alibi_slopes, return_softmax=return_softmax and dropout_p > 0, block_table=block_table)
     if is_grad:
         ctx.save_for_backward(q, k, v, out_padded, lse, cu_q, cu_k, rng)
         ctx.dropout_p, ctx.max_seqlen_q, ctx.max_seqlen_k = dropout_p, max_q, max_k
@@ -211,10 +240,17 @@ def _varlen_backward(ctx, dout):
     q, k, v, out, lse, cu_q, cu_k, rng = ctx.saved_tensors
     dout, q, k, v, out, og = _pad_bwd_headdim(dout, q, k, v, out)
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    _wrapped_flash_attn_varlen_backward(dout, q, k, v, out, lse, dq, dk, dv, cu_q, cu_k, ctx.max_seqlen_q,
-                                        ctx.max_seqlen_k, ctx.dropout_p, ctx.softmax_scale, ctx.causal,
-                                        ctx.window_size[0], ctx.window_size[1], ctx.softcap, ctx.alibi_slopes,
-                                        ctx.deterministic, rng_state=rng)
+    if (_scalars_ok(ctx.dropout_p, ctx.softmax_scale, ctx.causal, ctx.window_size, ctx.softcap) and type(ctx.deterministic) is bool
+            and type(ctx.max_seqlen_q) is int and type(ctx.max_seqlen_k) is int
+            and _plain(dout, q, k, v, out, lse, dq, dk, dv, cu_q, cu_k, ctx.alibi_slopes)):
+        _ext._bwd_common(maybe_contiguous(dout), maybe_contiguous(q), maybe_contiguous(k), maybe_contiguous(v), maybe_contiguous(out),
+                         lse, dq, dk, dv, ctx.alibi_slopes, ctx.dropout_p, ctx.softmax_scale, ctx.causal, ctx.window_size[0],
+                         ctx.window_size[1], ctx.softcap, ctx.deterministic, cu_q, cu_k, ctx.max_seqlen_q, ctx.max_seqlen_k)
+    else:
+        _wrapped_flash_attn_varlen_backward(dout, q, k, v, out, lse, dq, dk, dv, cu_q, cu_k, ctx.max_seqlen_q,
+                                            ctx.max_seqlen_k, ctx.dropout_p, ctx.softmax_scale, ctx.causal,
+                                            ctx.window_size[0], ctx.window_size[1], ctx.softcap, ctx.alibi_slopes,
+                                            ctx.deterministic, rng_state=rng)
     return dq[..., :og], dk[..., :og], dv[..., :og]
 
 

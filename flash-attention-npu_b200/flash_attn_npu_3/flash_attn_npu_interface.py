@@ -11,6 +11,8 @@ from typing import Optional, Tuple, Union
 import torch
 import torch.nn.functional as F
 
+from fa_b200_capi import plain as _plain
+from flash_attn_npu import flash_attn_npu as _v2_ext
 from . import flash_attn_npu_3 as _ext
 
 
@@ -32,9 +34,49 @@ def round_up_headdim(head_size: int) -> int:
 
 def _pad_bwd_headdim(dout, q, k, v, out):
     og = dout.size(-1)
-    target = round_multiple(max(t.size(-1) for t in (dout, q, k, v, out)), 64)
+    target = round_multiple(max(t.size(-1) for t in (dout, q, k, v, out)), 8)     # the kernels take any multiple of 8
     pad = lambda t: t if t.size(-1) == target else F.pad(t, [0, target - t.size(-1)])  # noqa: E731
     return pad(dout), pad(q), pad(k), pad(v), pad(out), og
+
+
+def _forward_body(q, k, v, k_new, v_new, qv, out_, cu_seqlens_q, cu_seqlens_k, cu_seqlens_k_new, seqused_q, seqused_k,
+                  max_seqlen_q, max_seqlen_k, page_table, kv_batch_idx, leftpad_k, rotary_cos, rotary_sin, seqlens_rotary,
+                  q_descale, k_descale, v_descale, softmax_scale, causal, window_size_left, window_size_right,
+                  attention_chunk, softcap, rotary_interleaved, scheduler_metadata, num_splits, pack_gqa, sm_margin):
+    q, k, k_new, v_new = [maybe_contiguous(x) for x in (q, k, k_new, v_new)]
+    v = v.contiguous() if v.stride(-1) != 1 else v
+    cu_seqlens_q, cu_seqlens_k, seqused_k, page_table, kv_batch_idx = [
+        maybe_contiguous(x) for x in (cu_seqlens_q, cu_seqlens_k, seqused_k, page_table, kv_batch_idx)]
+    return _ext.fwd(
+        q, k, v, k_new, v_new, qv, out_, cu_seqlens_q, cu_seqlens_k, cu_seqlens_k_new, seqused_q, seqused_k,
+        max_seqlen_q, max_seqlen_k, page_table, kv_batch_idx, leftpad_k, rotary_cos, rotary_sin, seqlens_rotary,
+        q_descale, k_descale, v_descale, softmax_scale, causal, window_size_left, window_size_right,
+        attention_chunk, softcap, rotary_interleaved, scheduler_metadata, num_splits, pack_gqa, sm_margin)
+
+
+def _direct(tensors, floats, ints, optional_ints, bools):
+    """Whether a custom op may be bypassed: its dispatch would do nothing but call the body, and the scalars have exactly the
+    schema's types, so that nothing would be converted or refused (see the v2 module for what this saves)."""
+    return (all(type(x) is float for x in floats) and all(type(x) is int for x in ints) and all(type(x) is bool for x in bools)
+            and all(x is None or type(x) is int for x in optional_ints)
+            and all(t is None or isinstance(t, torch.Tensor) for t in tensors) and _plain(*tensors))
+
+
+def _forward(q, k, v, k_new=None, v_new=None, qv=None, cu_seqlens_q=None, cu_seqlens_k=None, cu_seqlens_k_new=None, seqused_q=None,
+             seqused_k=None, max_seqlen_q=None, max_seqlen_k=None, page_table=None, kv_batch_idx=None, leftpad_k=None,
+             rotary_cos=None, rotary_sin=None, seqlens_rotary=None, q_descale=None, k_descale=None, v_descale=None,
+             softmax_scale=None, causal=False, window_size=(-1, -1), attention_chunk=0, softcap=0.0, rotary_interleaved=True,
+             scheduler_metadata=None, num_splits=1, pack_gqa=None, sm_margin=0):
+    """(out, lse) or (out, lse, out_accum, lse_accum) of the forward op."""
+    args = (q, k, v, k_new, v_new, qv, None, cu_seqlens_q, cu_seqlens_k, cu_seqlens_k_new, seqused_q, seqused_k,
+            max_seqlen_q, max_seqlen_k, page_table, kv_batch_idx, leftpad_k, rotary_cos, rotary_sin, seqlens_rotary,
+            q_descale, k_descale, v_descale, softmax_scale, causal, window_size[0], window_size[1], attention_chunk, softcap,
+            rotary_interleaved, scheduler_metadata, num_splits, pack_gqa, sm_margin)
+    if pack_gqa in (None, False, True) and _direct(args[:12] + args[14:23] + (scheduler_metadata,), (softmax_scale, softcap),
+                                                   (window_size[0], window_size[1], attention_chunk, num_splits, sm_margin),
+                                                   (max_seqlen_q, max_seqlen_k), (causal, rotary_interleaved)):
+        return _forward_body(*args)
+    return _flash_attn_forward(*args)
 
 
 @torch.library.custom_op("flash_attn_npu_3::_flash_attn_forward", mutates_args=(), device_types="cuda")
@@ -58,11 +100,7 @@ def _flash_attn_forward(
     scheduler_metadata: Optional[torch.Tensor] = None, num_splits: int = 1,
     pack_gqa: Optional[bool] = None, sm_margin: int = 0,
 ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
-    q, k, k_new, v_new = [maybe_contiguous(x) for x in (q, k, k_new, v_new)]
-    v = v.contiguous() if v.stride(-1) != 1 else v
-    cu_seqlens_q, cu_seqlens_k, seqused_k, page_table, kv_batch_idx = [
-        maybe_contiguous(x) for x in (cu_seqlens_q, cu_seqlens_k, seqused_k, page_table, kv_batch_idx)]
-    out, lse, out_accum, lse_accum = _ext.fwd(
+    out, lse, out_accum, lse_accum = _forward_body(
         q, k, v, k_new, v_new, qv, out_, cu_seqlens_q, cu_seqlens_k, cu_seqlens_k_new, seqused_q, seqused_k,
         max_seqlen_q, max_seqlen_k, page_table, kv_batch_idx, leftpad_k, rotary_cos, rotary_sin, seqlens_rotary,
         q_descale, k_descale, v_descale, softmax_scale, causal, window_size_left, window_size_right,
@@ -129,9 +167,14 @@ def _run_backward(ctx, dout, q, k, v, out, lse, cu_q=None, cu_k=None, max_q=None
     assert ctx.attention_chunk == 0, "backward does not support attention_chunk"
     dout, q, k, v, out, og = _pad_bwd_headdim(dout, q, k, v, out)
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    _flash_attn_backward(dout, q, k, v, out, lse, cu_q, cu_k, None, None, max_q, max_k, dq, dk, dv,
-                         ctx.softmax_scale, ctx.causal, ctx.window_size[0], ctx.window_size[1], ctx.softcap,
-                         ctx.deterministic, ctx.sm_margin)
+    if _direct((dout, q, k, v, out, lse, cu_q, cu_k, dq, dk, dv), (ctx.softmax_scale, ctx.softcap),
+               (ctx.window_size[0], ctx.window_size[1], ctx.sm_margin), (max_q, max_k), (ctx.causal, ctx.deterministic)):
+        _v2_ext._bwd_common(*[maybe_contiguous(x) for x in (dout, q, k, v, out)], lse, dq, dk, dv, None, 0.0, ctx.softmax_scale,
+                            ctx.causal, ctx.window_size[0], ctx.window_size[1], ctx.softcap, ctx.deterministic, cu_q, cu_k, max_q, max_k)
+    else:
+        _flash_attn_backward(dout, q, k, v, out, lse, cu_q, cu_k, None, None, max_q, max_k, dq, dk, dv,
+                             ctx.softmax_scale, ctx.causal, ctx.window_size[0], ctx.window_size[1], ctx.softcap,
+                             ctx.deterministic, ctx.sm_margin)
     return dq[..., :og], dk[..., :og], dv[..., :og]
 
 
@@ -147,10 +190,9 @@ class FlashAttnFunc(torch.autograd.Function):
                 deterministic=False, sm_margin=0, return_softmax=False, scheduler_metadata=None):
         if softmax_scale is None:
             softmax_scale = (q.shape[-1] + (qv.shape[-1] if qv is not None else 0)) ** (-0.5)
-        out, lse, *_ = _flash_attn_forward(
-            q, k, v, None, None, qv, None, None, None, None, None, None, None, None, None, None, None, None, None,
-            None, q_descale, k_descale, v_descale, softmax_scale, causal=causal, window_size_left=window_size[0],
-            window_size_right=window_size[1], attention_chunk=attention_chunk, softcap=softcap,
+        out, lse, *_ = _forward(
+            q, k, v, qv=qv, q_descale=q_descale, k_descale=k_descale, v_descale=v_descale, softmax_scale=softmax_scale,
+            causal=causal, window_size=window_size, attention_chunk=attention_chunk, softcap=softcap,
             scheduler_metadata=scheduler_metadata, num_splits=num_splits, pack_gqa=pack_gqa, sm_margin=sm_margin)
         ctx.save_for_backward(q, k, v, out, lse)
         _stash(ctx, softmax_scale, causal, window_size, attention_chunk, softcap, deterministic, sm_margin)
@@ -171,12 +213,11 @@ class FlashAttnVarlenFunc(torch.autograd.Function):
                 deterministic=False, sm_margin=0, return_softmax=False, scheduler_metadata=None):
         if softmax_scale is None:
             softmax_scale = (q.shape[-1] + (qv.shape[-1] if qv is not None else 0)) ** (-0.5)
-        out, lse, *_ = _flash_attn_forward(
-            q, k, v, None, None, qv, None, cu_seqlens_q, cu_seqlens_k, None, seqused_q, seqused_k, max_seqlen_q,
-            max_seqlen_k, None, None, None, None, None, None, q_descale, k_descale, v_descale, softmax_scale,
-            causal=causal, window_size_left=window_size[0], window_size_right=window_size[1],
-            attention_chunk=attention_chunk, softcap=softcap, scheduler_metadata=scheduler_metadata,
-            num_splits=num_splits, pack_gqa=pack_gqa, sm_margin=sm_margin)
+        out, lse, *_ = _forward(
+            q, k, v, qv=qv, cu_seqlens_q=cu_seqlens_q, cu_seqlens_k=cu_seqlens_k, seqused_q=seqused_q, seqused_k=seqused_k,
+            max_seqlen_q=max_seqlen_q, max_seqlen_k=max_seqlen_k, q_descale=q_descale, k_descale=k_descale, v_descale=v_descale,
+            softmax_scale=softmax_scale, causal=causal, window_size=window_size, attention_chunk=attention_chunk, softcap=softcap,
+            scheduler_metadata=scheduler_metadata, num_splits=num_splits, pack_gqa=pack_gqa, sm_margin=sm_margin)
         ctx.save_for_backward(q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k)
         ctx.max_seqlen_q, ctx.max_seqlen_k = max_seqlen_q, max_seqlen_k
         _stash(ctx, softmax_scale, causal, window_size, attention_chunk, softcap, deterministic, sm_margin)
@@ -203,10 +244,9 @@ class FlashAttnQKVPackedFunc(torch.autograd.Function):
             q, k, v = qkv.split([num_heads_q, hk, hk], dim=-2)
         if softmax_scale is None:
             softmax_scale = q.shape[-1] ** (-0.5)
-        out, lse, *_ = _flash_attn_forward(
-            q, k, v, None, None, None, None, None, None, None, None, None, None, None, None, None, None, None, None,
-            None, q_descale, k_descale, v_descale, softmax_scale, causal=causal, window_size_left=window_size[0],
-            window_size_right=window_size[1], attention_chunk=attention_chunk, softcap=softcap, sm_margin=sm_margin)
+        out, lse, *_ = _forward(
+            q, k, v, q_descale=q_descale, k_descale=k_descale, v_descale=v_descale, softmax_scale=softmax_scale, causal=causal,
+            window_size=window_size, attention_chunk=attention_chunk, softcap=softcap, sm_margin=sm_margin)
         ctx.save_for_backward(q, k, v, out, lse)
         ctx.ndim = qkv.dim()
         _stash(ctx, softmax_scale, causal, window_size, attention_chunk, softcap, deterministic, sm_margin)
@@ -284,14 +324,14 @@ def flash_attn_with_kvcache(q, k_cache, v_cache, k=None, v=None, qv=None, rotary
     if cache_seqlens is not None and isinstance(cache_seqlens, int):
         nb = q.shape[0] if cu_seqlens_q is None else cu_seqlens_q.numel() - 1
         cache_seqlens = torch.full((nb,), cache_seqlens, dtype=torch.int32, device=k_cache.device)
-    out, lse, *rest = _flash_attn_forward(
-        q, k_cache, v_cache, k, v, qv, None, cu_seqlens_q, None, cu_seqlens_k_new, None, cache_seqlens,
-        max_seqlen_q, None, page_table, cache_batch_idx, cache_leftpad, rotary_cos, rotary_sin, rotary_seqlens,
-        q_descale, k_descale, v_descale, softmax_scale, causal=causal, window_size_left=window_size[0],
-        window_size_right=window_size[1], attention_chunk=attention_chunk, softcap=softcap,
-        rotary_interleaved=rotary_interleaved, scheduler_metadata=scheduler_metadata, num_splits=num_splits,
-        pack_gqa=pack_gqa, sm_margin=sm_margin)
-    return (out, lse, *rest) if return_softmax_lse else out
+    out, lse, *rest = _forward(
+        q, k_cache, v_cache, k, v, qv, cu_seqlens_q, None, cu_seqlens_k_new, None, cache_seqlens, max_seqlen_q, None,
+        page_table, cache_batch_idx, cache_leftpad, rotary_cos, rotary_sin, rotary_seqlens, q_descale, k_descale, v_descale,
+        softmax_scale, causal, window_size, attention_chunk, softcap, rotary_interleaved, scheduler_metadata, num_splits,
+        pack_gqa, sm_margin)
+    if not return_softmax_lse:
+        return out
+    return (out, lse, *(torch.empty((0,), device=out.device) if x is None else x for x in rest))
 
 
 def get_scheduler_metadata(batch_size, max_seqlen_q, max_seqlen_k, num_heads_q, num_heads_kv, headdim,
