@@ -25,27 +25,35 @@ __device__ int g_fwd_sm100_error = 0;
 // vice versa.  The running max used as exponent base is only moved when the true max has grown by
 // more than 2^8 (the accumulator is rescaled then), so rescaling O is rare and stays in the
 // softmax warps.
+//
+// DUAL: calls whose query blocks have at most 128 rows.  There is no second query tile; both score buffers, both softmax
+// groups and both accumulators work on the SAME rows, group A on the even key tiles and group B on the odd ones, and the two
+// partial results are merged in the epilogue.  With one tile in flight the K and V stream stood still while that tile went
+// through QK^T, softmax and PV.
 // =================================================================================================
-template <int D>
+template <int D, bool DUAL>
 struct FwdSm100Smem2 {
     static constexpr int kSub = 128 * 128;
     static constexpr int kQ = (D / 64) * kSub;              // one query tile
     static constexpr int kKV = (D / 64) * kSub;
-    static constexpr int oQ = 0;                            // 2 tiles
-    static constexpr int oK = oQ + 2 * kQ;                  // 2 stages
-    static constexpr int oV = oK + 2 * kKV;                 // 2 stages
-    static constexpr int oBar = oV + 2 * kKV;
-    static constexpr int kBytes = oBar + 320;        // barriers and flags
+    static constexpr int kStages = DUAL ? 3 : 2;            // K and V buffers; the second Q tile's room goes to a third of each
+    static constexpr int oQ = 0;                            // 1 or 2 tiles
+    static constexpr int oK = oQ + (DUAL ? 1 : 2) * kQ;
+    static constexpr int oV = oK + kStages * kKV;
+    static constexpr int oBar = oV + kStages * kKV;         // barriers and flags
+    static constexpr int kBytes = oBar + 320;
+    static_assert(kBytes + 1024 <= 232448, "shared memory limit of a CTA");
 };
 
 #ifndef FA_FWD_POLY
 #define FA_FWD_POLY 2      // pairs of every 8 whose exponential runs on the FMA pipe
 #endif
-enum { C_Q = 0, C_KF0, C_KF1, C_KE0, C_KE1, C_VF0, C_VF1, C_VE0, C_VE1, C_SA, C_SB, C_PA, C_PB, C_PA2, C_PB2, C_OA, C_OB, C_DRAIN, C_COUNT };
+enum { C_Q = 0, C_KF0, C_KF1, C_KF2, C_KE0, C_KE1, C_KE2, C_VF0, C_VF1, C_VF2, C_VE0, C_VE1, C_VE2, C_SA, C_SB, C_PA, C_PB, C_PA2, C_PB2, C_OA, C_OB, C_DRAIN, C_COUNT };
 
-template <typename T, int D, bool BIAS>
+template <typename T, int D, bool BIAS, bool DUAL>
 __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constant__ Sm100FwdArgs a) {
-    using L = FwdSm100Smem2<D>;
+    using L = FwdSm100Smem2<D, DUAL>;
+    constexpr int NST = L::kStages;
     constexpr int NSUB = D / 64;
     constexpr int KSTEPS = D / 16;
     constexpr uint32_t TMEM_COLS = 512;
@@ -91,12 +99,12 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
     if (a.seqused_k) {                                       // cache call: the length lives on the device
         sk = (int)max(0LL, min((long long)a.seqused_k[b] + a.s_new, (long long)a.sk));   // an oversized entry is truncated to the capacity
     }
-    const int m0 = mblk * 2 * qpt;                           // first query position of the CTA
+    const int m0 = mblk * (DUAL ? 1 : 2) * qpt;              // first query position of the CTA
     if (m0 >= sq) return;
     if (g_fwd_sm100_error) return;
     const int wl = a.wl, wr = a.causal ? 0 : a.wr;
-    const int rows_cta = min(256, (sq - m0) * gq);           // tile rows in use
-    const bool has_b = rows_cta > 128;
+    const int rows_cta = min(DUAL ? 128 : 256, (sq - m0) * gq);          // tile rows in use
+    const bool has_b = !DUAL && rows_cta > 128;
 
     int lo_first, hi_first, lo_last, hi_last;
     window_bounds(m0, sq, sk, wl, wr, lo_first, hi_first);
@@ -188,7 +196,7 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
             const int kbatch = a.cu_q ? 0 : (a.cache_batch_idx ? a.cache_batch_idx[b] : b);
             bool ok = true;
             for (int j = 0; j < ntiles && ok; ++j) {
-                const int st = j & 1, use = j >> 1;
+                const int st = DUAL ? (int)((unsigned)j % NST) : j & 1, use = DUAL ? (int)((unsigned)j / NST) : j >> 1;
                 int krow = (a.cu_q ? k_off : 0) + (t_lo + j) * 128, kouter = kbatch;
                 int krow2 = 0, kouter2 = 0;                       // second half of the tile when it is copied in two boxes of 64 rows
                 if (btab) {
@@ -241,6 +249,45 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
                 return true;
             };
             bool ok = mbar_wait(bar(C_Q), 0, abort_flag, err, 3);
+            if constexpr (DUAL) {
+                // stale V rows, as in the other form below
+                auto clear_stale = [&](int j, int st) {
+                    if (!a.seqused_k || (t_lo + j) * 128 + 128 <= sk) return;
+                    const int first = max(0, sk - (t_lo + j) * 128);
+                    const int last = a.block_table ? 128 : min(128, a.sk - (t_lo + j) * 128);
+#pragma unroll
+                    for (int sub = 0; sub < NSUB; ++sub)
+                        for (int idx = first * 8 + lane; idx < last * 8; idx += 32)     // 16-byte chunks of rows first .. last - 1
+                            *reinterpret_cast<uint4*>(sgen + L::oV + st * L::kKV + sub * L::kSub + idx * 16) = make_uint4(0, 0, 0, 0);
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                };
+                // key tile j goes through score buffer and accumulator j & 1
+                auto scores = [&](int j) -> bool {
+                    if (!mbar_wait(bar(C_KF0 + j % NST), (j / NST) & 1, abort_flag, err, 7)) return false;
+                    tc_fence_after();
+                    umma_ss_scores<KSTEPS, L::kSub>(tmem + (j & 1) * 128, dQ0, umma_desc_at(dK0, (j % NST) * L::kKV), IDESC_QK);
+                    umma_commit_w(bar(C_SA + (j & 1)));
+                    umma_commit_w(bar(C_KE0 + j % NST));
+                    return true;
+                };
+                if (ok) ok = scores(0);
+                if (ok && ntiles > 1) ok = scores(1);
+                for (int j = 0; j < ntiles && ok; ++j) {
+                    const int x = j & 1, st = j % NST;
+                    ok = mbar_wait(bar(C_VF0 + st), (j / NST) & 1, abort_flag, err, 6);
+                    if (!ok) break;
+                    clear_stale(j, st);
+                    ok = mbar_wait(bar(C_PA + x), (j >> 1) & 1, abort_flag, err, 5);
+                    if (!ok) break;
+                    tc_fence_after();
+                    ok = issue_pv(x, st, j >> 1);
+                    if (!ok) break;
+                    umma_commit_w(bar(C_VE0 + st));
+                    if (j + 2 < ntiles) ok = scores(j + 2);
+                    else umma_commit_w(bar(C_OA + x));
+                }
+            } else {
             if (ok) ok = mbar_wait(bar(C_KF0), 0, abort_flag, err, 4);
             if (ok) {
                 tc_fence_after();
@@ -298,6 +345,7 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
                     umma_commit_w(bar(C_OB));
                 }
             }
+            }
             // The release of the last K/V stage has no waiter, and with one query tile in use it is issued after the
             // commit the epilogue waits for.  An arrive that the tensor core performs after the CTA has left would land
             // in shared memory the CTA no longer owns.  Commits complete in issue order, so the warp waits for a last
@@ -310,31 +358,32 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
     }
     } else {
     reg_alloc<224>();
-    if (warp < 4 || has_b) {
-        // ---------------------------------------------------------------- softmax of tile x
+    if (warp < 4 || has_b || DUAL) {
+        // ---------------------------------------------------------------- softmax of tile x (DUAL: of key tiles x, x + 2, ..)
         const int x = warp >> 2;
         const int r = tid & 127;
+        const int x0 = DUAL ? 0 : x * 128;                       // first tile row of this group
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const uint32_t t_s = tmem + lane_base + x * 128;
         const uint32_t t_o = tmem + lane_base + 256 + x * 128;
-        const int rows = min(128, rows_cta - x * 128);
-        const int qi = m0 + (x * 128 + r) / gq;                  // query position of this thread's row
+        const int rows = min(128, rows_cta - x0);
+        const int qi = m0 + (x0 + r) / gq;                  // query position of this thread's row
         int klo = 1, khi = 0;
         if (r < rows) window_bounds(qi, sq, sk, wl, wr, klo, khi);
         int lo_l, hi_f, tmp;
-        window_bounds(m0 + x * qpt, sq, sk, wl, wr, tmp, hi_f);
-        window_bounds(m0 + (x * 128 + rows - 1) / gq, sq, sk, wl, wr, lo_l, tmp);
+        window_bounds(m0 + x0 / gq, sq, sk, wl, wr, tmp, hi_f);
+        window_bounds(m0 + (x0 + rows - 1) / gq, sq, sk, wl, wr, lo_l, tmp);
         float m_used = -INFINITY, l_run = 0.f;
         // BIAS instantiation: the scores are turned into their final log2-domain values in registers (softcap, then
         // alibi, as the general kernel and the golden do), and the softmax below runs with a unit scale
         const float sc = BIAS ? 1.f : a.scale_log2;
         const float cap_out = a.softcap * kLog2e;
-        const float slope = (BIAS && a.alibi) ? a.alibi[(int64_t)b * a.alibi_sb + h0 + (x * 128 + r) % gq] * kLog2e : 0.f;
+        const float slope = (BIAS && a.alibi) ? a.alibi[(int64_t)b * a.alibi_sb + h0 + (x0 + r) % gq] * kLog2e : 0.f;
         const float rel = (float)(qi + sk - sq);                 // alibi distance of key j is |rel - j|
         bool ok = true;
-        const int nt_x = x == 0 ? nt0 : ntiles;
+        const int nt_x = DUAL ? (ntiles + 1 - x) / 2 : x == 0 ? nt0 : ntiles;
         for (int j = 0; j < nt_x && ok; ++j) {
-            const int n0 = (t_lo + j) * 128;
+            const int n0 = (t_lo + (DUAL ? 2 * j + x : j)) * 128;
             ok = mbar_wait(bar(C_SA + x), j & 1, abort_flag, err, 9);
             if (!ok) break;
             tc_fence_after();
@@ -441,17 +490,45 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
             const float s0 = sum_a.x + sum_b.x, s1 = sum_a.y + sum_b.y;
             l_run += s0 + s1;
         }
-        if (ok) ok = mbar_wait(bar(C_OA + x), 0, abort_flag, err, 10);
+        if (ok) ok = mbar_wait(bar(DUAL ? (int)C_OA : C_OA + x), 0, abort_flag, err, 10);
+        float f_a = 1.f, f_b = 0.f;                              // DUAL: weights of the two groups' results
+        if constexpr (DUAL) {
+            // All MMAs are done, so every copy has landed and been read: the exponent bases and row sums of both groups go
+            // through the K buffers.
+            if (ok && ntiles > 1) ok = mbar_wait(bar(C_OB), 0, abort_flag, err, 12);
+            float* merge = reinterpret_cast<float*>(sgen + L::oK);
+            merge[x * 256 + r] = m_used;
+            merge[x * 256 + 128 + r] = l_run;
+            asm volatile("barrier.cta.sync 1, 256;" ::: "memory");               // both groups, whatever became of their waits
+            const float m_a = merge[r], m_b = merge[256 + r];
+            m_used = fmaxf(m_a, m_b);
+            f_a = m_a == -INFINITY ? 0.f : ex2_approx(m_a - m_used);
+            f_b = m_b == -INFINITY ? 0.f : ex2_approx(m_b - m_used);
+            l_run = merge[128 + r] * f_a + merge[384 + r] * f_b;
+        }
         if (ok) {
             tc_fence_after();
             const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-            T* orow = out_row(x * 128 + r);
-            float* prow = a.nsplit > 1 ? a.o_part + part_row(x * 128 + r) * a.d : nullptr;
+            T* orow = out_row(x0 + r);
+            float* prow = a.nsplit > 1 ? a.o_part + part_row(x0 + r) * a.d : nullptr;
+            // DUAL: each group merges and stores one half of the columns
 #pragma unroll
-            for (int c = 0; c < D / 32; ++c) {
+            for (int cc = 0; cc < (DUAL ? D / 64 : D / 32); ++cc) {
+                const int c = DUAL ? x * (D / 64) + cc : cc;
                 uint32_t oreg[32];
-                tmem_ld32(t_o + c * 32, oreg);
+                tmem_ld32((DUAL ? t_o - x * 128 : t_o) + c * 32, oreg);
                 tmem_wait_ld();
+                if constexpr (DUAL) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * f_a);
+                    if (ntiles > 1) {                            // group B has worked: its accumulator holds something
+                        uint32_t ob[32];
+                        tmem_ld32(t_o + (1 - x) * 128 + c * 32, ob);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) oreg[i] = __float_as_uint(fmaf(__uint_as_float(ob[i]), f_b, __uint_as_float(oreg[i])));
+                    }
+                }
                 if (r < rows && prow) {
 #pragma unroll
                     for (int v = 0; v < 8; ++v)
@@ -470,8 +547,9 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
                     }
                 }
             }
-            if (r < rows && prow) a.lse_part[part_row(x * 128 + r)] = l_run > 0.f ? (m_used + log2f(l_run)) * kLn2 : -INFINITY;
-            else if (r < rows && a.lse) *lse_slot(x * 128 + r) = l_run > 0.f ? (m_used + log2f(l_run)) * kLn2 : INFINITY;
+            if (DUAL && x) {
+            } else if (r < rows && prow) a.lse_part[part_row(x0 + r)] = l_run > 0.f ? (m_used + log2f(l_run)) * kLn2 : -INFINITY;
+            else if (r < rows && a.lse) *lse_slot(x0 + r) = l_run > 0.f ? (m_used + log2f(l_run)) * kLn2 : INFINITY;
         }
     }
     }
@@ -932,11 +1010,11 @@ int grid_chunk(int64_t pairs, int64_t bytes_per_pair) {
     return (int)(c < 1 ? 1 : c);
 }
 
-template <typename T, int D, bool BIAS>
+template <typename T, int D, bool BIAS, bool DUAL>
 static int launch_sm100_b(const fa_fwd_params& p, Sm100FwdArgs& a) {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(p.stream);
-    auto kern = fwd_sm100_kernel2<T, D, BIAS>;
-    const int smem = FwdSm100Smem2<D>::kBytes + 1024;
+    auto kern = fwd_sm100_kernel2<T, D, BIAS, DUAL>;
+    const int smem = FwdSm100Smem2<D, DUAL>::kBytes + 1024;
     if (int e = cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute")) return e;
     const int qpc = 256 / a.gq;                              // query positions of a CTA
     const unsigned nbx = (unsigned)(((p.sq + qpc - 1) / qpc) * a.nsplit);
@@ -949,7 +1027,10 @@ static int launch_sm100_b(const fa_fwd_params& p, Sm100FwdArgs& a) {
 }
 template <typename T, int D>
 static int launch_sm100_t(const fa_fwd_params& p, Sm100FwdArgs& a) {
-    return (p.softcap > 0.f || p.alibi_slopes) ? launch_sm100_b<T, D, true>(p, a) : launch_sm100_b<T, D, false>(p, a);
+    const bool bias = p.softcap > 0.f || p.alibi_slopes;
+    // no query block has more than 128 rows
+    if ((long)p.sq * a.gq <= 128) return bias ? launch_sm100_b<T, D, true, true>(p, a) : launch_sm100_b<T, D, false, true>(p, a);
+    return bias ? launch_sm100_b<T, D, true, false>(p, a) : launch_sm100_b<T, D, false, false>(p, a);
 }
 template <typename T, int D, bool BIAS>
 static int launch_sm100_wide_b(const fa_fwd_params& p, Sm100FwdArgs& a) {
