@@ -69,6 +69,31 @@ static int check_common(const fa_fwd_params& p) {
     return FA_OK;
 }
 
+// Key splits of a prefill chunk: none, as many as one wave of CTAs holds, or `most` (about two waves).  The lengths are not known here, so each count is rated by the mean of two
+// estimates in microseconds, every sequence as long as the capacity (whole waves of CTAs) and lengths spread below it (0.6
+// of the keys, and the longest sequence at least); both with what a split costs, 6 us to start and finish a CTA and the
+// partials' way to memory and back.  A larger count has to be rated 5 % better.  Measured, 512 new tokens, H32/8 D128: B4
+// up to 16000 keys 238 us unsplit, 278 with two splits (which two waves of CTAs asked for); B1 16000 keys 224 / 138 / 153
+// us with one / two / four; B6 S300 H16 up to 32000 keys 542 / 428 with one / two.  Counts between one wave and `most` are
+// not tried: a second wave that is mostly empty made them the worst (B4 S128 up to 30000 keys: 150 / 160 / 132 us with one /
+// two / three).
+static int prefill_splits(const fa_fwd_params& p, long ctas, int most) {
+    const double sms = sm_count(), tiles = (p.sk + 127) / 128;
+    const double whole = tiles * (ctas * 256 <= (long)p.b * p.sq * p.hq * 2 ? 1.9 : 1.0);        // a CTA over all keys: two query tiles or one
+    const double rows = (double)p.b * p.sq * p.hq;
+    int best = 1;
+    double best_us = 0;
+    for (int n = 1; n <= most; ++n) {
+        if (n > 1 && n < most && ctas * n > (long)sms) continue;
+        const double one = whole / n, waves = (double)((long)((ctas * n + (long)sms - 1) / (long)sms));
+        const double spread = 0.6 * ctas * whole / sms + 0.25 * one;
+        const double cost = ctas * n / sms * 6.0 + (n > 1 ? rows * p.d * 8.0 * n / 4e6 + 5.0 : 0.0);
+        const double us = 0.5 * (waves * one + (spread > one ? spread : one)) + cost;
+        if (n == 1 || us < 0.95 * best_us) { best = n; best_us = us; }
+    }
+    return best;
+}
+
 void plan_forward(const fa_fwd_params& p, FwdPlan& plan) {
     memset(&plan, 0, sizeof(plan));
     const int G = p.hq / p.hkv;
@@ -92,7 +117,7 @@ void plan_forward(const fa_fwd_params& p, FwdPlan& plan) {
         const int min_keys = p.sq >= 64 ? 2048 : 512;
         const long cap = (p.sk + min_keys - 1) / min_keys;
         if (n > cap) n = cap;
-        nsplit = (int)(n < 1 ? 1 : n);
+        nsplit = p.sq >= 64 && n > 1 ? prefill_splits(p, ctas, (int)n) : (int)(n < 1 ? 1 : n);
     } else if (p.num_splits == 0 && plan.use_decode && nblocks > 1) {
         // decode kernel: the unit of parallelism is a warp per (sequence, KV head, split); aim at about
         // 1024 keys per split, at least four waves of warps, and never fewer than 256 keys per split
