@@ -3,7 +3,7 @@
 //
 // With the cap the softmax, not the tensor core, bounds the kernel: tanh by its exponential and a division makes three
 // special-function operations a score.  The two-tile kernel (fwd_sm100.cu), two softmax warps a scheduler with 128 scores
-// a thread and the cap branch on every score, took 432 us at B1 S8192 H16/8 D128 window 1024 bf16; this one 144.  What
+// a thread and the cap branch on every score, took 432 us at B1 S8192 H16/8 D128 window 1024 bf16; this one 135.  What
 // makes the difference:
 //  - two threads share a score row (64 scores each: warps 0-3 keys 0-63 of the tile, warps 4-7 keys 64-127), so that four
 //    softmax warps of two independent CTAs run on each scheduler, and the start and the end of a CTA run beside the other's
@@ -418,6 +418,7 @@ __global__ void __launch_bounds__(320, 2) fwd_single_sm100_kernel(const __grid_c
             };
             if (full && small) exp_phase(std::true_type{}, std::false_type{});
             else if (full) exp_phase(std::false_type{}, std::false_type{});
+            else if (small) exp_phase(std::true_type{}, std::true_type{});
             else exp_phase(std::false_type{}, std::true_type{});
             l_run += (sum_a.x + sum_b.x) + (sum_a.y + sum_b.y);
         }
