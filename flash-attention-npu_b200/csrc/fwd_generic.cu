@@ -658,9 +658,16 @@ __global__ void __launch_bounds__(256) combine_few_kernel(
 #pragma unroll
     for (int s = 0; s < NS; ++s) m = fmaxf(m, ls[s]);
     const float ms = m == -INFINITY ? 0.f : m;
-    float tot = 0.f;
+    // summed in the order of the warp reduction above (and of the peer-memory combine), so that the results are the same bits
+    float e[NS];
 #pragma unroll
-    for (int s = 0; s < NS; ++s) tot += expf(ls[s] - ms);
+    for (int s = 0; s < NS; ++s) e[s] = expf(ls[s] - ms);
+#pragma unroll
+    for (int d = NS / 2; d > 0; d >>= 1) {
+#pragma unroll
+        for (int s = 0; s < d; ++s) e[s] += e[s + d];
+    }
+    const float tot = e[0];
     const float l = tot > 0.f ? ms + logf(tot) : -INFINITY;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
