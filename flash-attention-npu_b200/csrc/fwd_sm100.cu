@@ -45,9 +45,11 @@ struct FwdSm100Smem2 {
     static_assert(kBytes + 1024 <= 232448, "shared memory limit of a CTA");
 };
 
-#ifndef FA_FWD_POLY
-#define FA_FWD_POLY 2      // pairs of every 8 whose exponential runs on the FMA pipe
-#endif
+// Pairs of every 8 whose exponential runs on the FMA pipe.  The special-function unit is not the limiter and the
+// polynomial costs six times the instructions, so a few are enough.  Head dim 128: 1 of 8 against 2 and 0, packed causal
+// prefill of the benchmark under the power cap 3841 / 3916 / 3869 us.  Head dim 64, full attention B1 S8192 H37: 814 us with
+// 2, 859 with 1, 858 with 3.
+template <int D> constexpr int kFwdPoly = D == 128 ? 1 : 2;
 enum { C_Q = 0, C_KF0, C_KF1, C_KF2, C_KE0, C_KE1, C_KE2, C_VF0, C_VF1, C_VF2, C_VE0, C_VE1, C_VE2, C_SA, C_SB, C_PA, C_PB, C_PA2, C_PB2, C_OA, C_OB, C_DRAIN, C_COUNT };
 
 template <typename T, int D, bool BIAS, bool DUAL>
@@ -81,6 +83,7 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
     // lost 20 % at 128 pairs of 2 MiB).  Pairs past the end of the last chunk leave.
     const int pair = blockIdx.z * a.chunk + blockIdx.x;
     if (pair >= a.b * a.nheads_grid) return;
+    const int failed = g_fwd_sm100_error;                    // in flight beside the lengths below
     const uint3 bi = make_uint3(blockIdx.y, pair % a.nheads_grid, pair / a.nheads_grid);   // (query block x split, head, batch entry)
     const int nbx = gridDim.y;
     const int b = bi.z;
@@ -101,7 +104,7 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
     }
     const int m0 = mblk * (DUAL ? 1 : 2) * qpt;              // first query position of the CTA
     if (m0 >= sq) return;
-    if (g_fwd_sm100_error) return;
+    if (failed) return;
     const int wl = a.wl, wr = a.causal ? 0 : a.wr;
     const int rows_cta = min(DUAL ? 128 : 256, (sq - m0) * gq);          // tile rows in use
     const bool has_b = !DUAL && rows_cta > 128;
@@ -154,12 +157,59 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
         return;
     }
 
-    if (tid == 0) {
-        for (int i = 0; i < C_COUNT; ++i) mbar_init(bar(i), (i >= C_PA && i <= C_PB2) ? 128u : 1u);
-        *abort_flag = 0;
-        mbar_fence_init();
-    }
+    const int qrow0 = (a.cu_q ? q_off : 0) + m0;
+    const int qb = a.cu_q ? 0 : b;
+    // where key tile j lives: (row, outermost coordinate) of the K / V maps.  Dense and packed operands: row
+    // in the batch entry; cache: row in the cache entry of this batch; paged cache: row inside the page
+    // that the page table names (a tile never straddles pages when the page size is a multiple of 128; pages of
+    // an odd multiple of 64 tokens are copied in two boxes of 64 rows, each from its own page)
+    const int32_t* btab = a.block_table ? a.block_table + (int64_t)b * a.bt_stride : nullptr;
+    auto place = [&](int j, int& krow, int& kouter, int& krow2, int& kouter2) {
+        krow = (a.cu_q ? k_off : 0) + (t_lo + j) * 128;
+        kouter = a.cu_q ? 0 : (a.cache_batch_idx ? a.cache_batch_idx[b] : b);
+        krow2 = 0; kouter2 = 0;                              // second half of the tile when it is copied in two boxes of 64 rows
+        if (btab) {
+            const int pos = (t_lo + j) * 128;
+            kouter = btab[pos / a.page_size];
+            krow = pos % a.page_size;
+            if (a.kv_box == 64) {
+                // the tile may end in the next page; a half past the table's end is never attended (its
+                // columns are masked by the length), it is read from the first half's page
+                const bool in_table = (pos + 64) / a.page_size < a.bt_stride;
+                kouter2 = in_table ? btab[(pos + 64) / a.page_size] : kouter;
+                krow2 = in_table ? (pos + 64) % a.page_size : krow;
+            }
+        }
+    };
+    auto load = [&](const CUtensorMap* map, uint32_t dst, uint32_t full, int krow, int kouter, int krow2, int kouter2) {
+        mbar_expect_tx(full, L::kKV);
+#pragma unroll
+        for (int s = 0; s < NSUB; ++s) {
+            tma_load_4d(dst + s * L::kSub, map, full, s * 64, hk, krow, kouter);
+            if (a.kv_box == 64) tma_load_4d(dst + s * L::kSub + 64 * 128, map, full, s * 64, hk, krow2, kouter2);
+        }
+    };
     if (warp == 8) {
+        // The copy warp sets up the barriers and asks for Q and the first K and V before anything else, so that they are on
+        // their way while tensor memory is allocated and the other warps arrive.
+        if (lane == 0) {
+            tma_prefetch_desc(&a.tq); tma_prefetch_desc(&a.tk); tma_prefetch_desc(&a.tv);
+            for (int i = 0; i < C_COUNT; ++i) mbar_init(bar(i), (i >= C_PA && i <= C_PB2) ? 128u : 1u);
+            *abort_flag = 0;
+            mbar_fence_init();
+            mbar_expect_tx(bar(C_Q), has_b ? 2 * L::kQ : L::kQ);
+#pragma unroll
+            for (int s = 0; s < NSUB; ++s) tma_load_4d(sQ + s * L::kSub, &a.tq, bar(C_Q), s * 64, h0, qrow0, qb);
+            int krow, kouter, krow2, kouter2;
+            place(0, krow, kouter, krow2, kouter2);
+            load(&a.tk, sK, bar(C_KF0), krow, kouter, krow2, kouter2);
+            if (has_b) {
+#pragma unroll
+                for (int s = 0; s < NSUB; ++s) tma_load_4d(sQ + L::kQ + s * L::kSub, &a.tq, bar(C_Q), s * 64, h0, qrow0 + qpt, qb);
+            }
+            load(&a.tv, sV, bar(C_VF0), krow, kouter, krow2, kouter2);
+        }
+        __syncwarp();
         tmem_alloc(smem_addr(tmem_slot), TMEM_COLS);
         tmem_relinquish();
     }
@@ -168,8 +218,6 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     int* err = &g_fwd_sm100_error;
-    const int qrow0 = (a.cu_q ? q_off : 0) + m0;
-    const int qb = a.cu_q ? 0 : b;
 
     // Register file split by warp group: the copy/MMA group (warps 8-11, of which 10 and 11 only
     // exist to complete the group) keeps 56 registers a thread, the two softmax groups take 224.  The sum
@@ -180,53 +228,17 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
     reg_dealloc<56>();
     if (warp == 8) {
         if (lane == 0) {
-            tma_prefetch_desc(&a.tq); tma_prefetch_desc(&a.tk); tma_prefetch_desc(&a.tv);
-            mbar_expect_tx(bar(C_Q), has_b ? 2 * L::kQ : L::kQ);
-#pragma unroll
-            for (int s = 0; s < NSUB; ++s) tma_load_4d(sQ + s * L::kSub, &a.tq, bar(C_Q), s * 64, h0, qrow0, qb);
-            if (has_b) {
-#pragma unroll
-                for (int s = 0; s < NSUB; ++s) tma_load_4d(sQ + L::kQ + s * L::kSub, &a.tq, bar(C_Q), s * 64, h0, qrow0 + qpt, qb);
-            }
-            // where key tile j lives: (row, outermost coordinate) of the K / V maps.  Dense and packed operands: row
-            // in the batch entry; cache: row in the cache entry of this batch; paged cache: row inside the page
-            // that the page table names (a tile never straddles pages when the page size is a multiple of 128; pages of
-            // an odd multiple of 64 tokens are copied in two boxes of 64 rows, each from its own page)
-            const int32_t* btab = a.block_table ? a.block_table + (int64_t)b * a.bt_stride : nullptr;
-            const int kbatch = a.cu_q ? 0 : (a.cache_batch_idx ? a.cache_batch_idx[b] : b);
             bool ok = true;
-            for (int j = 0; j < ntiles && ok; ++j) {
+            for (int j = 1; j < ntiles && ok; ++j) {
                 const int st = DUAL ? (int)((unsigned)j % NST) : j & 1, use = DUAL ? (int)((unsigned)j / NST) : j >> 1;
-                int krow = (a.cu_q ? k_off : 0) + (t_lo + j) * 128, kouter = kbatch;
-                int krow2 = 0, kouter2 = 0;                       // second half of the tile when it is copied in two boxes of 64 rows
-                if (btab) {
-                    const int pos = (t_lo + j) * 128;
-                    kouter = btab[pos / a.page_size];
-                    krow = pos % a.page_size;
-                    if (a.kv_box == 64) {
-                        // the tile may end in the next page; a half past the table's end is never attended (its
-                        // columns are masked by the length), it is read from the first half's page
-                        const bool in_table = (pos + 64) / a.page_size < a.bt_stride;
-                        kouter2 = in_table ? btab[(pos + 64) / a.page_size] : kouter;
-                        krow2 = in_table ? (pos + 64) % a.page_size : krow;
-                    }
-                }
+                int krow, kouter, krow2, kouter2;
+                place(j, krow, kouter, krow2, kouter2);
                 if (use > 0) ok = mbar_wait(bar(C_KE0 + st), (use - 1) & 1, abort_flag, err, 1);
                 if (!ok) break;
-                mbar_expect_tx(bar(C_KF0 + st), L::kKV);
-#pragma unroll
-                for (int s = 0; s < NSUB; ++s) {
-                    tma_load_4d(sK + st * L::kKV + s * L::kSub, &a.tk, bar(C_KF0 + st), s * 64, hk, krow, kouter);
-                    if (a.kv_box == 64) tma_load_4d(sK + st * L::kKV + s * L::kSub + 64 * 128, &a.tk, bar(C_KF0 + st), s * 64, hk, krow2, kouter2);
-                }
+                load(&a.tk, sK + st * L::kKV, bar(C_KF0 + st), krow, kouter, krow2, kouter2);
                 if (use > 0) ok = mbar_wait(bar(C_VE0 + st), (use - 1) & 1, abort_flag, err, 2);
                 if (!ok) break;
-                mbar_expect_tx(bar(C_VF0 + st), L::kKV);
-#pragma unroll
-                for (int s = 0; s < NSUB; ++s) {
-                    tma_load_4d(sV + st * L::kKV + s * L::kSub, &a.tv, bar(C_VF0 + st), s * 64, hk, krow, kouter);
-                    if (a.kv_box == 64) tma_load_4d(sV + st * L::kKV + s * L::kSub + 64 * 128, &a.tv, bar(C_VF0 + st), s * 64, hk, krow2, kouter2);
-                }
+                load(&a.tv, sV + st * L::kKV, bar(C_VF0 + st), krow, kouter, krow2, kouter2);
             }
         }
     } else if (warp == 9) {
@@ -485,7 +497,7 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel2(const __grid_constan
                 }
             };
             // masked tiles keep the special-function path: it maps -inf to an exact zero
-            if (full) exp_phase(std::integral_constant<int, FA_FWD_POLY>{});
+            if (full) exp_phase(std::integral_constant<int, kFwdPoly<D>>{});
             else exp_phase(std::integral_constant<int, 0>{});
             const float s0 = sum_a.x + sum_b.x, s1 = sum_a.y + sum_b.y;
             l_run += s0 + s1;
@@ -873,7 +885,7 @@ __global__ void __launch_bounds__(384, 1) fwd_sm100_kernel_wide(const __grid_con
                     mbar_arrive(bar((hlf ? W_P0B : W_P0) + buf));
                 }
             };
-            if (full) exp_phase(std::integral_constant<int, FA_FWD_POLY>{});
+            if (full) exp_phase(std::integral_constant<int, kFwdPoly<D>>{});
             else exp_phase(std::integral_constant<int, 0>{});
             l_run += (sum_a.x + sum_b.x) + (sum_a.y + sum_b.y);
         }
