@@ -19,6 +19,7 @@
 // Math and rounding points as in bwd_sm100.cu (fag_kernel.cpp:400-465, fag_epilogue_op.hpp:1287-1322, :1394,
 // :1447-1480, fag_epilogue_post.hpp:149-200).  No atomics, fixed order of sums; all waits are bounded.
 #include "bwd_sm100_common.cuh"
+#include "bwd_wide_tiles.h"
 
 namespace fa {
 
@@ -36,7 +37,6 @@ int bwd_wide_error_flag(bool clear) {
 namespace {
 
 constexpr int kSub = 128 * 128;                              // bytes of a [128 rows x 64 columns] sub-tile
-constexpr size_t kTileBytes = 128 * 128 * 2;                 // one stored P^T or dS^T tile
 
 struct alignas(64) WideBwdArgs {
     CUtensorMap tq, tdo, tk, tv;
@@ -49,14 +49,14 @@ struct alignas(64) WideBwdArgs {
     const int32_t* cu_k;
     int b, sq, sk, hq, hkv, d;           // d: the call's head dim, a multiple of 8 (tile copies zero-fill the columns past it)
     float scale, scale_log2;
-    int causal, wl, wr;
+    WideGrid grid;                       // blocks a head and the masks that say which of them meet
     float softcap, cap_in2, cap_out;     // as in Sm100BwdArgs
     const float* alibi;
     int64_t alibi_sb;
     // stored tiles of the (batch entry, KV head) pairs unit0 .. of this launch: tile (pair, head of the group, key block,
     // query block) = 128 keys x 128 queries as [16 chunks of 8 queries][128 keys][8 queries]
     unsigned char *p_tiles, *ds_tiles;
-    int unit0, nkb, nqb, steps_per_cta;
+    int unit0, steps_per_cta;
 };
 
 struct Geometry {
@@ -64,21 +64,7 @@ struct Geometry {
     __device__ Geometry(const WideBwdArgs& a, int unit) : b(unit / a.hkv), hk(unit % a.hkv), q_off(0), k_off(0), sq(a.sq), sk(a.sk) {
         if (a.cu_q) { q_off = a.cu_q[b]; sq = a.cu_q[b + 1] - q_off; k_off = a.cu_k[b]; sk = a.cu_k[b + 1] - k_off; }
     }
-    // query blocks [lo, hi) that key block n is visible to: the one rule both kernels go by
-    __device__ void query_blocks(const WideBwdArgs& a, int n, int& lo, int& hi) const {
-        const int n0 = n * 128, krows = min(128, sk - n0), diff = sk - sq;
-        const int wl = a.wl, wr = a.causal ? 0 : a.wr;
-        int i_lo = 0, i_hi = sq - 1;
-        if (wr >= 0) i_lo = max(0, n0 - diff - wr);
-        if (wl >= 0) i_hi = min(sq - 1, n0 + krows - 1 + wl - diff);
-        lo = i_lo / 128;
-        hi = n0 < sk && i_hi >= i_lo ? i_hi / 128 + 1 : lo;
-    }
 };
-
-__device__ __forceinline__ size_t tile_at(const WideBwdArgs& a, int local_unit, int g, int n, int m) {
-    return ((((size_t)local_unit * (a.hq / a.hkv) + g) * a.nkb + n) * a.nqb + m) * kTileBytes;
-}
 
 // ------------------------------------------------------------------------------------------------------
 // Scores.  K and V of the key block stay in shared memory; Q and dO arrive as [128 x 64] sub-tiles through one ring
@@ -121,11 +107,10 @@ __global__ void __launch_bounds__(608, 1) bwd_wide_scores_kernel(const __grid_co
     if (n0 >= sk) return;
     if (g_bwd_wide_error) return;
     const int G = a.hq / a.hkv;
-    const int wl = a.wl, wr = a.causal ? 0 : a.wr;
+    const int wl = a.grid.wl, wr = a.grid.causal ? 0 : a.grid.wr;
     const int diff = sk - sq;
-    int mb_lo, mb_hi;
-    geo.query_blocks(a, nb, mb_lo, mb_hi);
-    const int nmb = mb_hi - mb_lo;
+    const BlockRange qr = wide_query_blocks(a.grid, sq, sk, nb);
+    const int mb_lo = qr.lo, nmb = qr.hi - qr.lo;
     const int s_begin = blockIdx.z * a.steps_per_cta;
     const int steps = min(nmb * G - s_begin, a.steps_per_cta);
     if (steps <= 0) return;
@@ -242,7 +227,7 @@ __global__ void __launch_bounds__(608, 1) bwd_wide_scores_kernel(const __grid_co
             __syncwarp();
             if (s + 1 < steps) fetch_vec(s + 1, st_l, st_d);
             // thread's 16-byte chunk of chunk row c: 8 queries of key r (a warp stores 512 contiguous bytes)
-            const size_t off = tile_at(a, local, g, nb, m) + ((size_t)(cg * 4) * 128 + r) * 16;
+            const size_t off = wide_tile_at(a.grid, G, local, g, nb, m) + ((size_t)(cg * 4) * 128 + r) * 16;
             uint4* p_dst = reinterpret_cast<uint4*>(a.p_tiles + off);
             uint4* ds_dst = reinterpret_cast<uint4*>(a.ds_tiles + off);
             ok = mbar_wait(bar(WB_S0 + buf), (s >> 1) & 1, abort_flag, err, 66);
@@ -334,7 +319,7 @@ enum { GB_F0 = 0, GB_F1, GB_E0, GB_E1, GB_ACC, GB_COUNT };
 template <int D>
 struct GradSmem {
     static constexpr int kRows = (D / 64) * kSub;
-    static constexpr int kStage = (int)kTileBytes + kRows;
+    static constexpr int kStage = (int)kWideTileBytes + kRows;
     static constexpr int kBytes = 2 * kStage + 8 * GB_COUNT + 16;
 };
 
@@ -364,26 +349,22 @@ __global__ void __launch_bounds__(192, 1) bwd_wide_grads_kernel(const __grid_con
     if (g_bwd_wide_error) return;
 
     // mode 0: dV, 1: dK, 2: dQ
-    const bool is_q = (int)blockIdx.y >= 2 * a.nkb;
+    const bool is_q = (int)blockIdx.y >= 2 * a.grid.nkb;
     const int mode = is_q ? 2 : (int)(blockIdx.y & 1);
-    int g_q = 0, blk, lo, hi, steps;
+    int g_q = 0, blk, steps;
+    BlockRange br;                                           // query blocks (dV, dK) or key blocks (dQ) that are summed over
     if (!is_q) {
         blk = blockIdx.y >> 1;
         if (blk * 128 >= sk) return;
-        geo.query_blocks(a, blk, lo, hi);
-        steps = (hi - lo) * G;
+        br = wide_query_blocks(a.grid, sq, sk, blk);
+        steps = (br.hi - br.lo) * G;
     } else {
-        const int y = blockIdx.y - 2 * a.nkb;
+        const int y = blockIdx.y - 2 * a.grid.nkb;
         g_q = y % G;
-        blk = a.nqb - 1 - y / G;
+        blk = a.grid.nqb - 1 - y / G;
         if (blk * 128 >= sq) return;
-        lo = a.nkb; hi = 0;                                  // the key blocks that reach this query block form one range
-        for (int n = 0; n * 128 < sk; ++n) {
-            int ml, mh;
-            geo.query_blocks(a, n, ml, mh);
-            if (blk >= ml && blk < mh) { lo = min(lo, n); hi = max(hi, n + 1); }
-        }
-        steps = max(0, hi - lo);
+        br = wide_key_blocks(a.grid, sq, sk, blk);
+        steps = max(0, br.hi - br.lo);
     }
     const int rows = min(128, (is_q ? sq : sk) - blk * 128);
     T* out;
@@ -421,17 +402,17 @@ __global__ void __launch_bounds__(192, 1) bwd_wide_grads_kernel(const __grid_con
             bool ok = true;
             for (int j = 0; j < steps && ok; ++j) {
                 const int st = j & 1;
-                const int g = is_q ? g_q : j / (hi - lo);
-                const int other = lo + (is_q ? j : j % (hi - lo));            // query block (dV, dK) or key block (dQ)
-                const size_t tile = is_q ? tile_at(a, local, g, other, blk) : tile_at(a, local, g, blk, other);
+                const int g = is_q ? g_q : j / (br.hi - br.lo);
+                const int other = br.lo + (is_q ? j : j % (br.hi - br.lo));
+                const size_t tile = is_q ? wide_tile_at(a.grid, G, local, g, other, blk) : wide_tile_at(a.grid, G, local, g, blk, other);
                 if (j >= 2) ok = mbar_wait(bar(GB_E0 + st), ((j >> 1) - 1) & 1, abort_flag, err, 71);
                 if (!ok) break;
                 const uint32_t s0 = sbase + st * L::kStage;
                 mbar_expect_tx(bar(GB_F0 + st), L::kStage);
-                bulk_load_1d(s0, tiles + tile, (uint32_t)kTileBytes, bar(GB_F0 + st));
+                bulk_load_1d(s0, tiles + tile, (uint32_t)kWideTileBytes, bar(GB_F0 + st));
 #pragma unroll
                 for (int c = 0; c < NSUB; ++c)
-                    tma_load_4d(s0 + (uint32_t)kTileBytes + c * kSub, map, bar(GB_F0 + st), c * 64, is_q ? hk : hk * G + g, row0 + other * 128, bb);
+                    tma_load_4d(s0 + (uint32_t)kWideTileBytes + c * kSub, map, bar(GB_F0 + st), c * 64, is_q ? hk : hk * G + g, row0 + other * 128, bb);
             }
         }
     } else if (warp == 1) {
@@ -442,7 +423,7 @@ __global__ void __launch_bounds__(192, 1) bwd_wide_grads_kernel(const __grid_con
             if (!ok) break;
             tc_fence_after();
             const uint32_t s0 = sbase + st * L::kStage;
-            const uint64_t dB = umma_desc(s0 + (uint32_t)kTileBytes, kSub, 1024);
+            const uint64_t dB = umma_desc(s0 + (uint32_t)kWideTileBytes, kSub, 1024);
             // Stored tile: element (key k, query q) at chunk (q / 8) x 2048 + k x 16 + (q % 8) x 2 bytes.
             if (!is_q) {
                 // K step = 16 queries = 2 chunks; along K the chunks lie 2048 bytes apart, along M eight keys are 128 bytes
@@ -490,7 +471,7 @@ constexpr size_t kWideGroupBytes = (size_t)128 << 20;
 constexpr size_t kWideWorkspaceLimit = (size_t)6 << 30;      // one KV head's tiles may take this much at most
 
 size_t unit_bytes(const fa_bwd_params& p) {                  // P^T and dS^T tiles of one (batch entry, KV head) pair
-    return (size_t)(p.hq / p.hkv) * ((p.sk + 127) / 128) * ((p.sq + 127) / 128) * 2 * kTileBytes;
+    return (size_t)(p.hq / p.hkv) * ((p.sk + 127) / 128) * ((p.sq + 127) / 128) * 2 * kWideTileBytes;
 }
 int64_t units_per_launch(const fa_bwd_params& p) {
     const int64_t units = (int64_t)p.b * p.hkv;
@@ -513,16 +494,16 @@ int launch_t(const fa_bwd_params& p, WideBwdArgs& a, cudaStream_t st) {
     // Query blocks a score CTA walks: long walks amortise its K and V (128 KiB against 128 KiB a step), short ones fill the
     // GPU: sixteen while that leaves two CTAs for three SMs (sixteen against about two CTAs an SM: 1002 against 1050 us at
     // B1 S8192 H8, 133 against 142 at B2 S2048 H8/4), fewer below.
-    const int64_t tiles = per * G * a.nkb * a.nqb / (p.causal ? 2 : 1);
+    const int64_t tiles = per * G * a.grid.nkb * a.grid.nqb / (p.causal ? 2 : 1);
     a.steps_per_cta = 16;
     while (a.steps_per_cta > 4 && tiles / a.steps_per_cta < sm_count() * 2 / 3) a.steps_per_cta /= 2;
-    const unsigned nz = (unsigned)(((int64_t)a.nqb * G + a.steps_per_cta - 1) / a.steps_per_cta);
+    const unsigned nz = (unsigned)(((int64_t)a.grid.nqb * G + a.steps_per_cta - 1) / a.steps_per_cta);
     for (int64_t u = 0; u < units; u += per) {
         const unsigned n = (unsigned)(units - u < per ? units - u : per);
         a.unit0 = (int)u;
-        k1<<<dim3(n, a.nkb, nz), 608, smem1, st>>>(a);
+        k1<<<dim3(n, a.grid.nkb, nz), 608, smem1, st>>>(a);
         mark_kernel(st);
-        k2<<<dim3(n, 2 * a.nkb + G * a.nqb), 192, smem2, st>>>(a);
+        k2<<<dim3(n, 2 * a.grid.nkb + G * a.grid.nqb), 192, smem2, st>>>(a);
         mark_kernel(st);
     }
     return cuda_ok(cudaGetLastError(), "bwd_wide launch");
@@ -570,10 +551,9 @@ int launch_bwd_wide_sm100(const fa_bwd_params& p) {
     a.cu_q = p.cu_seqlens_q; a.cu_k = p.cu_seqlens_k;
     a.b = p.b; a.sq = p.sq; a.sk = p.sk; a.hq = p.hq; a.hkv = p.hkv; a.d = p.d;
     a.scale = p.scale; a.scale_log2 = p.scale * kLog2e;
-    a.causal = p.causal; a.wl = p.window_left; a.wr = p.window_right;
+    a.grid = {(p.sk + 127) / 128, (p.sq + 127) / 128, p.causal, p.window_left, p.window_right};
     a.softcap = p.softcap; a.cap_in2 = p.softcap > 0.f ? 2.f * kLog2e * p.scale / p.softcap : 0.f; a.cap_out = p.softcap * kLog2e;
     a.alibi = p.alibi_slopes; a.alibi_sb = p.alibi_stride_b;
-    a.nkb = (p.sk + 127) / 128; a.nqb = (p.sq + 127) / 128;
     a.p_tiles = reinterpret_cast<unsigned char*>(p.workspace) + delta_bytes(p);
     a.ds_tiles = a.p_tiles + (size_t)units_per_launch(p) * (unit_bytes(p) / 2);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(p.stream);
