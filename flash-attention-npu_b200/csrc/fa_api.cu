@@ -4,6 +4,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include "error_flags.h"
 #include "fa_internal.h"
 
 namespace fa {
@@ -356,15 +357,17 @@ int fa_copy_2d_async(void* dst, size_t dst_pitch, const void* src, size_t src_pi
 const char* fa_last_error(void) { return g_err; }
 const char* fa_version(void) { return "fa_b200 0.1.0 (sm_100a)"; }
 const char* fa_last_kernel(void) { return g_kernel; }
+static int any_error_flag(bool clear) {
+    static int (*const flags[])(bool) = {fa::sm100_error_flag, fa::decode_error_flag};
+    return fa::first_error(flags, 2, clear);
+}
 void fa_debug_set(int key, int value) {
-    if (key == 3) { fa::sm100_error_flag(true); fa::decode_error_flag(true); }
+    if (key == 3) any_error_flag(true);
     if (key == 4) fa::decode_set_use_tma(value);
     if (key == 7) fa::bwd_sm100_set_ds_spill(value);
 }
 int fa_debug_get(int key) {
-    if (key != 2) return 0;
-    const int a = fa::sm100_error_flag(false);
-    return a ? a : fa::decode_error_flag(false);
+    return key == 2 ? any_error_flag(false) : 0;
 }
 void fa_set_kernel_events(void** events, int count) {
     g_events = reinterpret_cast<cudaEvent_t*>(events);

@@ -6,6 +6,7 @@
 // Every mbarrier wait is bounded; a timeout records a code in g_fwd_sm100_error and the CTA
 // frees its tensor memory and returns.
 #include "fwd_sm100_common.cuh"
+#include "error_flags.h"
 
 namespace fa {
 
@@ -1129,16 +1130,16 @@ int launch_fwd_sm100(const fa_fwd_params& p, int nsplit, int keys_per_split, flo
     return p.d <= 64 ? launch_sm100_t<__nv_bfloat16, 64>(p, a) : launch_sm100_t<__nv_bfloat16, 128>(p, a);
 }
 
-int sm100_error_flag(bool clear) {
+static int fwd_sm100_error_flag(bool clear) {
     int v = 0;
     cudaMemcpyFromSymbol(&v, g_fwd_sm100_error, sizeof(int));
     if (clear) { int z = 0; cudaMemcpyToSymbol(g_fwd_sm100_error, &z, sizeof(int)); }
-    int w = bwd_sm100_error_flag(clear);
-    const int w2 = bwd_wide_error_flag(clear);
-    if (!w) w = w2;
-    if (!w) w = fwd_single_error_flag(clear);
-    const int m = mla_pair_error_flag(clear);
-    return v ? v : (w ? w : m);
+    return v;
+}
+
+int sm100_error_flag(bool clear) {
+    static int (*const flags[])(bool) = {fwd_sm100_error_flag, bwd_sm100_error_flag, bwd_wide_error_flag, fwd_single_error_flag, mla_pair_error_flag};
+    return first_error(flags, sizeof(flags) / sizeof(flags[0]), clear);
 }
 
 }  // namespace fa
