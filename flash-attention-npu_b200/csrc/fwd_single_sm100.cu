@@ -216,10 +216,10 @@ __global__ void __launch_bounds__(320, 2) fwd_single_sm100_kernel(const __grid_c
                         krow2 = in_table ? (pos + 64) % a.page_size : krow;
                     }
                 }
-                if (use > 0) ok = mbar_wait(bar(N_KE0 + st), (use - 1) & 1, abort_flag, err, 61);
+                if (use > 0) ok = mbar_wait(bar(N_KE0 + st), (use - 1) & 1, abort_flag, err, 81);
                 if (!ok) break;
                 load(sK + st * L::kTile, &a.tk, bar(N_KF0 + st), krow, kouter, krow2, kouter2);
-                if (use > 0) ok = mbar_wait(bar(N_VE0 + st), (use - 1) & 1, abort_flag, err, 62);
+                if (use > 0) ok = mbar_wait(bar(N_VE0 + st), (use - 1) & 1, abort_flag, err, 82);
                 if (!ok) break;
                 load(sV + st * L::kTile, &a.tv, bar(N_VF0 + st), krow, kouter, krow2, kouter2);
             }
@@ -231,22 +231,22 @@ __global__ void __launch_bounds__(320, 2) fwd_single_sm100_kernel(const __grid_c
             umma_commit_w(bar(N_S));
             umma_commit_w(bar(N_KE0 + j % NST));
         };
-        bool ok = mbar_wait(bar(N_Q), 0, abort_flag, err, 63);
-        if (ok) ok = mbar_wait(bar(N_KF0), 0, abort_flag, err, 64);
+        bool ok = mbar_wait(bar(N_Q), 0, abort_flag, err, 83);
+        if (ok) ok = mbar_wait(bar(N_KF0), 0, abort_flag, err, 84);
         if (ok) { tc_fence_after(); issue_qk(0); }
         for (int j = 0; j < ntiles && ok; ++j) {
             const int st = j % NST;
             const bool more = j + 1 < ntiles;
             if (kOwnP && more) {                             // the next scores as soon as these have been read
-                ok = mbar_wait(bar(N_KF0 + (j + 1) % NST), ((j + 1) / NST) & 1, abort_flag, err, 67);
-                if (ok) ok = mbar_wait(bar(N_SR), j & 1, abort_flag, err, 68);
+                ok = mbar_wait(bar(N_KF0 + (j + 1) % NST), ((j + 1) / NST) & 1, abort_flag, err, 87);
+                if (ok) ok = mbar_wait(bar(N_SR), j & 1, abort_flag, err, 88);
                 if (!ok) break;
                 tc_fence_after();
                 issue_qk(j + 1);
             }
             // the copies are waited for first, so that only the MMAs stand between "P is ready" and the tensor core
-            ok = mbar_wait(bar(N_VF0 + st), (j / NST) & 1, abort_flag, err, 66);
-            if (!kOwnP && ok && more) ok = mbar_wait(bar(N_KF0 + (j + 1) % NST), ((j + 1) / NST) & 1, abort_flag, err, 67);
+            ok = mbar_wait(bar(N_VF0 + st), (j / NST) & 1, abort_flag, err, 86);
+            if (!kOwnP && ok && more) ok = mbar_wait(bar(N_KF0 + (j + 1) % NST), ((j + 1) / NST) & 1, abort_flag, err, 87);
             if (!ok) break;
             if (a.seqused_k && (t_lo + j) * 128 + 128 > sk) {
                 // cache rows past the sequence may hold NaN patterns and 0 x NaN is NaN: the V rows that the copy fetched
@@ -260,13 +260,13 @@ __global__ void __launch_bounds__(320, 2) fwd_single_sm100_kernel(const __grid_c
                 fence_proxy_async_smem();
                 __syncwarp();
             }
-            ok = mbar_wait(bar(N_P0), j & 1, abort_flag, err, 65);
+            ok = mbar_wait(bar(N_P0), j & 1, abort_flag, err, 85);
             if (!ok) break;
             tc_fence_after();
             // 16 keys = 8 columns of P and 2048 bytes of V a step; keys 0-31 and 64-95, then 32-63 and 96-127
             const uint64_t bv = umma_desc_at(dV, st * L::kTile);
             umma_ts_quad<0, 8, P_HALF, P_HALF + 8, 0, 128, 512, 640>(tmem + COL_O, tmem + COL_P, bv, IDESC_PV, j > 0);
-            ok = mbar_wait(bar(N_P1), j & 1, abort_flag, err, 71);
+            ok = mbar_wait(bar(N_P1), j & 1, abort_flag, err, 91);
             if (!ok) break;
             tc_fence_after();
             umma_ts_quad<16, 24, P_HALF + 16, P_HALF + 24, 256, 384, 768, 896>(tmem + COL_O, tmem + COL_P, bv, IDESC_PV, 1);
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(320, 2) fwd_single_sm100_kernel(const __grid_c
         // no arrive of a commit may land after the CTA has left: wait for a last one (see the two-tile kernel)
         if (ok) {
             umma_commit_w(bar(N_DRAIN));
-            ok = mbar_wait(bar(N_DRAIN), 0, abort_flag, err, 73);
+            ok = mbar_wait(bar(N_DRAIN), 0, abort_flag, err, 93);
         }
     } else {
         const int quarter = warp & 3, half = warp >> 2;
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(320, 2) fwd_single_sm100_kernel(const __grid_c
         bool ok = true;
         for (int j = 0; j < ntiles; ++j) {
             const int n0 = (t_lo + j) * 128 + half * 64;     // first key of this thread's 64
-            ok = ok && mbar_wait(bar(N_S), j & 1, abort_flag, err, 69);
+            ok = ok && mbar_wait(bar(N_S), j & 1, abort_flag, err, 89);
             tc_fence_after();
             // warp-uniform: every row of the warp sees every key / no row sees any key of chunk c
             const bool full = n0 >= all_lo && n0 + 63 <= all_hi;
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(320, 2) fwd_single_sm100_kernel(const __grid_c
                 if (m_used == -INFINITY) m_used = m_row;
                 if (j > 0 && __any_sync(0xffffffffu, m_row > m_used + kRescaleThreshold)) {
                     if constexpr (kOwnP) {                   // P V of the last tile may still be running
-                        ok = ok && mbar_wait(bar(N_PV), (j - 1) & 1, abort_flag, err, 72);
+                        ok = ok && mbar_wait(bar(N_PV), (j - 1) & 1, abort_flag, err, 92);
                         tc_fence_after();
                     }
                     const float m_next = fmaxf(m_used, m_row);
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(320, 2) fwd_single_sm100_kernel(const __grid_c
                         });
                     }
                     if (kOwnP && c == 0 && j > 0) {          // P of the last tile has been read
-                        ok = ok && mbar_wait(bar(N_PV), (j - 1) & 1, abort_flag, err, 74);
+                        ok = ok && mbar_wait(bar(N_PV), (j - 1) & 1, abort_flag, err, 94);
                         tc_fence_after();
                     }
                     tmem_st16(t_p + c * 16, preg);
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(320, 2) fwd_single_sm100_kernel(const __grid_c
         s_sum[half * 128 + r] = l_run;
         ok = !pair_any(bid, !ok);
         const float l_tot = s_sum[r] + s_sum[128 + r];
-        if (ok) ok = mbar_wait(bar(N_O), 0, abort_flag, err, 70);
+        if (ok) ok = mbar_wait(bar(N_O), 0, abort_flag, err, 90);
         if (ok) {
             tc_fence_after();
             const float inv = l_tot > 0.f ? 1.f / l_tot : 0.f;

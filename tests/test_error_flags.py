@@ -40,3 +40,14 @@ def test_every_kernel_with_an_error_flag_is_asked():
     readers = {m for t in text.values() for m in re.findall(r"int (\w+_error_flag)\(bool clear\) \{", t)} - {"any_error_flag"}
     asked = {m for t in text.values() for lst in re.findall(r"flags\[\]\)\(bool\) = \{([^}]*)\}", t) for m in re.findall(r"\w+_error_flag", lst)}
     assert readers == asked and len(readers) >= 7
+
+
+def test_a_wait_code_belongs_to_one_kernel():
+    """Kernels whose flags are reported through one function number their waits apart (the latent decode's, older, overlap the
+    backward's)."""
+    seen = {}
+    for f in sorted(os.listdir(SRC)):
+        if f.endswith(".cu") and f != "mla_sm100_pair.cu":
+            for code in set(re.findall(r"err, (\d+)\)", open(os.path.join(SRC, f)).read())):
+                assert seen.setdefault(code, f) == f, (code, f, seen[code])
+    assert len(seen) >= 50
