@@ -318,11 +318,17 @@ def _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p
     dq = torch.empty_like(q) if dq_ is None else dq_
     dk = torch.empty_like(k) if dk_ is None else dk_
     dv = torch.empty_like(v) if dv_ is None else dv_
-    leaves = []
-    for t in (dout, q, k, v, out, dq, dk, dv):
+    leaves, copies = [], []
+    for i, t in enumerate((dout, q, k, v, out, dq, dk, dv)):
         s = t.stride()
         if s[-1] != 1:
             raise RuntimeError("Input tensor must have contiguous last dimension")
+        if i < 5 and (t.data_ptr() % 16 or min(s) <= 0 or (s[0] | s[1] | s[-2]) % 8):
+            # The caller of a backward does not choose how autograd lays out the gradient of the output (a slice of a
+            # concatenation, an expanded sum): what the 16-byte loads and tile copies cannot read in place is copied.
+            t = t.clone(memory_format=torch.contiguous_format)
+            copies.append(t)
+            s = t.stride()
         leaves += (t.data_ptr(), 0, s[0], s[1]) if packed else (t.data_ptr(), s[0], s[1], s[2])
     if packed:
         total_q, hq, _ = q.shape
@@ -357,7 +363,7 @@ def _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p
         ws = capi.workspace(capi._bwd_min_bytes(buf), device)
     capi.set_workspace(capi.BWD_BLOCK, buf, ws, ws.numel())
     capi.launch(capi._call_varlen_bwd if packed else capi._call_bwd, buf, device)
-    del keep
+    del keep, copies
     return dq, dk, dv
 
 
