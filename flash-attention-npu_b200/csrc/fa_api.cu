@@ -297,11 +297,13 @@ static int run_backward(const fa_bwd_params& pin) {
     if (p.window_right >= p.sq - 1) p.window_right = -1;
     mark_kernel(reinterpret_cast<cudaStream_t>(p.stream));
     const bool fast = g_policy == 0 && bwd_sm100_supported(p);
-    const bool wide = g_policy == 0 && bwd_wide_sm100_supported(p);
-    const size_t need = fast ? bwd_sm100_workspace_min(p) : wide ? bwd_wide_sm100_workspace(p) : bwd_generic_workspace(p);
+    const size_t need = fast ? bwd_sm100_workspace_min(p) : bwd_generic_workspace(p);
     if (!p.workspace || p.workspace_bytes < need)
         return fail(FA_ERR_WORKSPACE, "workspace of %zu bytes required, %zu given", need, p.workspace_bytes);
-    return fast ? launch_bwd_sm100(p) : wide ? launch_bwd_wide_sm100(p) : launch_bwd_generic(p);
+    if (fast) return launch_bwd_sm100(p);
+    // above head dim 128 the tcgen05 kernels need room for P and dS tiles (up to 6 GiB); without it the general kernels run
+    const bool wide = g_policy == 0 && bwd_wide_sm100_supported(p) && p.workspace_bytes >= bwd_wide_sm100_workspace(p);
+    return wide ? launch_bwd_wide_sm100(p) : launch_bwd_generic(p);
 }
 
 int fa_bwd(const fa_bwd_params* p) {
@@ -318,14 +320,15 @@ int fa_varlen_bwd(const fa_bwd_params* p) {
     return run_backward(*p);
 }
 
-static size_t bwd_workspace(const fa_bwd_params* p, size_t (*fast)(const fa_bwd_params&)) {
+static size_t bwd_workspace(const fa_bwd_params* p, bool least) {
     if (!p || p->hq <= 0) return 0;
-    if (bwd_wide_sm100_supported(*p)) return bwd_wide_sm100_workspace(*p);
-    const size_t a = bwd_generic_workspace(*p), b = fast(*p);
-    return a > b ? a : b;
+    const size_t general = bwd_generic_workspace(*p);
+    if (p->d > 128) return !least && bwd_wide_sm100_supported(*p) ? bwd_wide_sm100_workspace(*p) : general;
+    const size_t fast = least ? bwd_sm100_workspace_min(*p) : bwd_sm100_workspace(*p);
+    return general > fast ? general : fast;
 }
-size_t fa_bwd_workspace_bytes(const fa_bwd_params* p) { return bwd_workspace(p, bwd_sm100_workspace); }
-size_t fa_bwd_workspace_min_bytes(const fa_bwd_params* p) { return bwd_workspace(p, bwd_sm100_workspace_min); }
+size_t fa_bwd_workspace_bytes(const fa_bwd_params* p) { return bwd_workspace(p, false); }
+size_t fa_bwd_workspace_min_bytes(const fa_bwd_params* p) { return bwd_workspace(p, true); }
 
 int fa_combine(const fa_combine_params* c) {
     if (!c) return fail(FA_ERR_NULL, "params is null");

@@ -359,7 +359,7 @@ def _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p
         capi.raw_stream(device), alibi, alibi_sb)
     try:
         ws = capi.workspace(capi._bwd_bytes(buf), device)
-    except torch.OutOfMemoryError:                           # without room for the dS tiles the kernels recompute them
+    except torch.OutOfMemoryError:                           # without room for P and dS tiles the kernels recompute them
         ws = capi.workspace(capi._bwd_min_bytes(buf), device)
     capi.set_workspace(capi.BWD_BLOCK, buf, ws, ws.numel())
     capi.launch(capi._call_varlen_bwd if packed else capi._call_bwd, buf, device)

@@ -92,3 +92,46 @@ def test_wide_backward_over_several_launches(b, sq, sk, h, hkv, causal):
     for n, x, y, r in zip(("dq", "dk", "dv"), got, again, ref):
         assert torch.equal(x, y), n
         assert (x.float() - r.float()).abs().max().item() <= 3 * 2.0 ** -8 * r.float().abs().max().item(), n
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_wide_backward_without_room_for_the_tiles(packed, monkeypatch):
+    """The allocator refuses the workspace with the tiles: the call runs on the least one, with the general kernels' bits."""
+    import fa_b200_capi as capi
+    from flash_attn_npu import flash_attn_npu as ext
+    s, h, hkv, d = 600, 4, 2, 256
+    shape = (lambda n: (2 * s, n, d)) if packed else (lambda n: (2, s, n, d))
+    q, do = (torch.randn(*shape(h), device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(*shape(hkv), device="cuda").bfloat16() for _ in range(2))
+    cu = torch.tensor([0, s, 2 * s], dtype=torch.int32, device="cuda")
+    if packed:
+        out, lse, _, _ = ext.varlen_fwd(q, k, v, None, cu, cu, None, None, None, None, s, s, 0.0, 0.1, False, True, -1, -1, 0.0, False, None)
+    else:
+        out, lse, _, _ = ext.fwd(q, k, v, None, None, 0.0, 0.1, True, -1, -1, 0.0, False, None)
+
+    def run():
+        if packed:
+            g = ext.varlen_bwd(do, q, k, v, out, lse, None, None, None, cu, cu, None, s, s, 0.0, 0.1, False, True, -1, -1, 0.0, False, None, None)
+        else:
+            g = ext.bwd(do, q, k, v, out, lse, None, None, None, None, 0.0, 0.1, True, -1, -1, 0.0, False, None, None)
+        torch.cuda.synchronize()
+        return g[:3], capi.last_kernel()
+
+    assert run()[1] == "sm100_wide_tcgen05_bwd"
+    capi.lib.fa_set_kernel_policy(1)
+    try:
+        want, _ = run()
+    finally:
+        capi.lib.fa_set_kernel_policy(0)
+    real, sizes = capi.workspace, []
+
+    def small(n, device):
+        sizes.append(n)
+        if n > 1 << 20:
+            raise torch.OutOfMemoryError("no room")
+        return real(n, device)
+
+    monkeypatch.setattr(capi, "workspace", small)
+    got, name = run()
+    assert name == "generic_mma_bwd" and len(sizes) == 2 and sizes[1] < 1 << 20 < sizes[0]
+    assert all(torch.equal(x, y) for x, y in zip(got, want))
