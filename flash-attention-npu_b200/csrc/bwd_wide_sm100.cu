@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(608, 1) bwd_wide_scores_kernel(const __grid_co
             tmem_ld32(tmem + lane_base + COL_S + buf * 128 + cg * 32, pr);
             tmem_wait_ld();
             const bool inside = __all_sync(0xffffffffu, i0 >= qi_lo && i0 + 31 <= qi_hi);
+            auto seen = [&](int i) { return i0 + i >= qi_lo && i0 + i <= qi_hi; };
             float slope = 0.f;
             if constexpr (BIAS) { if (a.alibi) slope = a.alibi[(int64_t)b * a.alibi_sb + hk * G + g] * kLog2e; }
 #pragma unroll
@@ -267,11 +268,8 @@ __global__ void __launch_bounds__(608, 1) bwd_wide_scores_kernel(const __grid_co
                 float2 p01 = make_float2(ex2_approx(x01.x), ex2_approx(x01.y));
                 float2 p23 = make_float2(ex2_approx(x23.x), ex2_approx(x23.y));
                 if (!inside) {
-                    const int qi = i0 + i;
-                    p01.x = (qi >= qi_lo && qi <= qi_hi) ? p01.x : 0.f;
-                    p01.y = (qi + 1 >= qi_lo && qi + 1 <= qi_hi) ? p01.y : 0.f;
-                    p23.x = (qi + 2 >= qi_lo && qi + 2 <= qi_hi) ? p23.x : 0.f;
-                    p23.y = (qi + 3 >= qi_lo && qi + 3 <= qi_hi) ? p23.y : 0.f;
+                    p01 = make_float2(seen(i) ? p01.x : 0.f, seen(i + 1) ? p01.y : 0.f);
+                    p23 = make_float2(seen(i + 2) ? p23.x : 0.f, seen(i + 3) ? p23.y : 0.f);
                 }
                 pr[i] = __float_as_uint(p01.x * fac[0]); pr[i + 1] = __float_as_uint(p01.y * fac[1]);
                 pr[i + 2] = __float_as_uint(p23.x * fac[2]); pr[i + 3] = __float_as_uint(p23.y * fac[3]);
@@ -291,10 +289,16 @@ __global__ void __launch_bounds__(608, 1) bwd_wide_scores_kernel(const __grid_co
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
                 const float4 nd = *reinterpret_cast<const float4*>(vec + 32 + i);
-                const float2 d01 = mul2(make_float2(__uint_as_float(pr[i]), __uint_as_float(pr[i + 1])),
+                float2 d01 = mul2(make_float2(__uint_as_float(pr[i]), __uint_as_float(pr[i + 1])),
                                         add2(make_float2(__uint_as_float(dr[i]), __uint_as_float(dr[i + 1])), make_float2(nd.x, nd.y)));
-                const float2 d23 = mul2(make_float2(__uint_as_float(pr[i + 2]), __uint_as_float(pr[i + 3])),
+                float2 d23 = mul2(make_float2(__uint_as_float(pr[i + 2]), __uint_as_float(pr[i + 3])),
                                         add2(make_float2(__uint_as_float(dr[i + 2]), __uint_as_float(dr[i + 3])), make_float2(nd.z, nd.w)));
+                if (!inside) {
+                    // selected, not multiplied: the rows that a tile copy fetched past the end of a packed sequence are its
+                    // neighbour's, and 0 x NaN is NaN
+                    d01 = make_float2(seen(i) ? d01.x : 0.f, seen(i + 1) ? d01.y : 0.f);
+                    d23 = make_float2(seen(i + 2) ? d23.x : 0.f, seen(i + 3) ? d23.y : 0.f);
+                }
                 w[i / 2] = Elem<T>::pack(d01.x, d01.y);
                 w[i / 2 + 1] = Elem<T>::pack(d23.x, d23.y);
             }
@@ -423,6 +427,20 @@ __global__ void __launch_bounds__(192, 1) bwd_wide_grads_kernel(const __grid_con
             if (!ok) break;
             tc_fence_after();
             const uint32_t s0 = sbase + st * L::kStage;
+            if (a.cu_q) {
+                // rows past the end of a packed sequence are the next one's and meet zeros of the tile: cleared, so that a NaN
+                // or infinity stays in its own sequence (past the end of a dense batch entry the copy fills with zeros)
+                const int other = br.lo + (is_q ? j : j % (br.hi - br.lo));
+                const int first = (is_q ? sk : sq) - other * 128;
+                if (first < 128) {
+#pragma unroll
+                    for (int sub = 0; sub < NSUB; ++sub)
+                        for (int idx = first * 8 + lane; idx < 128 * 8; idx += 32)          // 16-byte chunks of rows first .. 127
+                            *reinterpret_cast<uint4*>(sgen + st * L::kStage + kWideTileBytes + sub * kSub + idx * 16) = make_uint4(0, 0, 0, 0);
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                }
+            }
             const uint64_t dB = umma_desc(s0 + (uint32_t)kWideTileBytes, kSub, 1024);
             // Stored tile: element (key k, query q) at chunk (q / 8) x 2048 + k x 16 + (q % 8) x 2 bytes.
             if (!is_q) {

@@ -135,3 +135,32 @@ def test_wide_backward_without_room_for_the_tiles(packed, monkeypatch):
     got, name = run()
     assert name == "generic_mma_bwd" and len(sizes) == 2 and sizes[1] < 1 << 20 < sizes[0]
     assert all(torch.equal(x, y) for x, y in zip(got, want))
+
+
+@pytest.mark.parametrize("d", [136, 256])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("causal,win,cap,alibi", [(True, (-1, -1), 0.0, False), (False, (-1, -1), 0.0, False), (False, (70, 40), 0.0, True), (True, (-1, -1), 3.0, False)])
+def test_non_finite_values_stay_in_their_packed_sequence(d, bad, causal, win, cap, alibi):
+    import fa_b200_capi as capi
+    from flash_attn_npu import flash_attn_npu as ext
+    lens, h, hkv = [200, 77, 130, 300], 4, 2
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    q, do = (torch.randn(sum(lens), h, d, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(sum(lens), hkv, d, device="cuda").bfloat16() for _ in range(2))
+    slopes = torch.rand(h, device="cuda") * 0.1 if alibi else None
+    tail = (cu, cu, slopes, 300, 300, 0.0, d ** -0.5, False, causal, *win, cap, False, None, None)
+    out, lse, _, _ = ext.varlen_fwd(q, k, v, None, cu, cu, None, None, None, slopes, 300, 300, 0.0, d ** -0.5, False, causal, *win, cap, False, None)
+
+    def run():
+        g = ext.varlen_bwd(do, q, k, v, out, lse, None, None, None, *tail)[:3]
+        torch.cuda.synchronize()
+        assert capi.last_kernel() == "sm100_wide_tcgen05_bwd" and capi.lib.fa_debug_get(2) == 0
+        return g
+
+    want = run()
+    for t in (q, k, v, do, out):
+        t[200:277] = bad
+    got = run()
+    for x, y in zip(got, want):
+        for s in (slice(0, 200), slice(277, None)):
+            assert torch.equal(x[s], y[s])
