@@ -164,3 +164,22 @@ def test_non_finite_values_stay_in_their_packed_sequence(d, bad, causal, win, ca
     for x, y in zip(got, want):
         for s in (slice(0, 200), slice(277, None)):
             assert torch.equal(x[s], y[s])
+
+
+@pytest.mark.parametrize("cap", [0.5, 30.0, 2e4, 1e6])
+def test_capped_scores_keep_their_precision(cap):
+    """A large cap multiplies whatever absolute error tanh has: with the oracle's LSE the gradients stay within the roundings of
+    P, dS and the result."""
+    import fa_b200_capi as capi
+    from flash_attn_npu import flash_attn_npu as ext
+    d, dt = 256, torch.float16
+    q, k, v, do = ((torch.rand(1, 260, 2, d) * 2 - 1).to(dt) for _ in range(4))
+    scale = d ** -0.5
+    out, lse = orc.attention_fwd(q.float(), k.float(), v.float(), scale, True, (-1, -1), cap, data_type=torch.float32)
+    lp = orc.attention_bwd(q, k, v, do, lse, scale, True, (-1, -1), cap)
+    f32 = orc.attention_bwd(q.float(), k.float(), v.float(), do.float(), lse, scale, True, (-1, -1), cap)
+    got = ext.bwd(*(t.cuda() for t in (do, q, k, v, out.to(dt), lse)), None, None, None, None, 0.0, scale, True, -1, -1, cap, False, None, None)[:3]
+    torch.cuda.synchronize()
+    assert capi.last_kernel() == "sm100_wide_tcgen05_bwd"
+    for n, g, a, r in zip(("dq", "dk", "dv"), got, lp, f32):
+        assert_within(n, g.cpu(), a, r, roundings=3)
