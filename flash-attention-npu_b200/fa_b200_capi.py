@@ -211,14 +211,18 @@ def set_workspace(block, buf, ws, nbytes):
     _POINTER(buf, block.offsets["workspace_bytes"], nbytes)
 
 
-def raw_stream(device):
-    """The current stream of `device` as an integer, without building a Stream object."""
-    return torch._C._cuda_getCurrentRawStream(device.index)
+if hasattr(torch._C, "_cuda_getCurrentRawStream"):
+    def raw_stream(device):
+        """The current stream of `device` as an integer, without building a Stream object."""
+        return torch._C._cuda_getCurrentRawStream(device.index)
+else:
+    def raw_stream(device):
+        return torch.cuda.current_stream(device).cuda_stream
 
 
 def launch(fn, buf, device):
     """Run an entry point with `device` current."""
-    if torch._C._cuda_getDevice() == device.index:
+    if torch.cuda.current_device() == device.index:
         check(fn(buf))
     else:
         with torch.cuda.device(device):
@@ -228,13 +232,34 @@ def launch(fn, buf, device):
 _PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 
+def _dispatch_state():
+    """-> a function that says whether anything stands between a call of a custom op and its CUDA kernel: tracing, modes,
+    functorch and forward-mode levels, an active profiler (which shows the op by its name).  The names it asks are torch's
+    own and not all public: where one is missing it always says yes, and every call takes the op."""
+    try:
+        profiling = torch.autograd._profiler_enabled
+        modes, functions = torch._C._len_torch_dispatch_stack, torch._C._len_torch_function_stack
+        functorch, tracing = torch._C._functorch.peek_interpreter_stack, torch._C._get_tracing_state
+        forward_ad = torch.autograd.forward_ad
+
+        def acting():
+            return (modes() or functions() or functorch() is not None or tracing() is not None
+                    or forward_ad._current_level >= 0 or profiling())
+
+        acting()
+        return acting
+    except AttributeError:
+        return lambda: True
+
+
+_dispatch_acts = _dispatch_state()
+
+
 def plain(*tensors):
     """True when dispatching a custom op with these arguments would do nothing but run its CUDA kernel, so that the caller may
-    run it itself: ordinary strided CUDA tensors, nothing tracing, compiling, transforming (functorch, forward-mode) or
-    intercepting calls (modes, subclasses, lazy negation), and nothing that autograd would have to record."""
-    if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
-            or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._get_tracing_state() is not None
-            or torch.autograd.forward_ad._current_level >= 0):
+    run it itself: ordinary strided CUDA tensors, nothing tracing, compiling, transforming (functorch, forward-mode),
+    profiling or intercepting calls (modes, subclasses, lazy negation), and nothing that autograd would have to record."""
+    if torch.compiler.is_compiling() or _dispatch_acts():
         return False
     grad = torch.is_grad_enabled()
     for t in tensors:

@@ -140,3 +140,33 @@ def test_transforms_behave_as_with_the_op(monkeypatch):
     here = kinds()
     monkeypatch.setattr(i2, "_plain", lambda *t: False)
     assert here == kinds()
+
+
+@pytest.mark.parametrize("name", ["_len_torch_dispatch_stack", "_len_torch_function_stack", "_get_tracing_state"])
+def test_a_torch_without_one_of_the_names_takes_the_op(name, monkeypatch):
+    assert not capi._dispatch_state()()
+    monkeypatch.delattr(torch._C, name)
+    acts = capi._dispatch_state()
+    monkeypatch.undo()
+    assert acts()
+
+
+def test_a_profiler_is_something_the_dispatch_acts_for():
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]):
+        assert capi._dispatch_acts()
+    assert not capi._dispatch_acts()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("version", [2, 3])
+def test_a_profiler_sees_the_ops(version):
+    import flash_attn_npu as fa2
+    import flash_attn_npu_3 as fa3
+    fa = fa2 if version == 2 else fa3
+    q, k, v, do = _inputs()
+    x = [t.requires_grad_(True) for t in (q, k, v)]
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        torch.autograd.grad(fa.flash_attn_func(*x), x, do)
+    names = {e.name for e in prof.events()}
+    pkg = "flash_attn_npu" if version == 2 else "flash_attn_npu_3"
+    assert {f"{pkg}::_flash_attn_forward", f"{pkg}::_flash_attn_backward"} <= names
