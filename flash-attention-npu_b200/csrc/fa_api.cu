@@ -11,6 +11,7 @@ namespace fa {
 
 static thread_local char g_err[512] = "";
 static thread_local const char* g_kernel = "";
+static thread_local int g_form = 0;
 static std::atomic<int> g_policy{0};          // process-wide test switch (fa_set_kernel_policy)
 // optional per-kernel timing: the caller lends CUDA events, one is recorded after every launch
 static thread_local cudaEvent_t* g_events = nullptr;
@@ -28,7 +29,7 @@ int fail(int code, const char* fmt, ...) {
     va_end(ap);
     return code;
 }
-void note_kernel(const char* name) { g_kernel = name; }
+void note_kernel(const char* name, int form) { g_kernel = name; g_form = form; }
 int cuda_ok(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return FA_OK;
     return fail(FA_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
@@ -370,6 +371,7 @@ void fa_debug_set(int key, int value) {
     if (key == 7) fa::bwd_sm100_set_ds_spill(value);
 }
 int fa_debug_get(int key) {
+    if (key == 8) return g_form;
     return key == 2 ? any_error_flag(false) : 0;
 }
 void fa_set_kernel_events(void** events, int count) {

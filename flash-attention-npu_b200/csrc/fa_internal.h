@@ -9,7 +9,14 @@ namespace fa {
 
 // error reporting (thread-local message, see fa_api.cu)
 int fail(int code, const char* fmt, ...);
-void note_kernel(const char* name);
+// The name that fa_last_kernel() reports, and which form of that kernel ran (fa_debug_get key 8): several forms share a name
+enum KernelForm {
+    FORM_USUAL = 0,
+    FORM_SHORT_QUERIES = 1,              // forward: both softmax groups on the same query rows
+    FORM_ONE_TILE = 2,                   // forward, capped scores: one query tile a CTA
+    FORM_STORED_DS = 3,                  // backward: dQ from stored dS tiles
+};
+void note_kernel(const char* name, int form = FORM_USUAL);
 int cuda_ok(cudaError_t e, const char* what);
 // records the next lent timing event (if any) on the stream; call after every kernel launch
 void mark_kernel(cudaStream_t st);

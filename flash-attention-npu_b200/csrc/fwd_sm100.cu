@@ -1038,11 +1038,12 @@ static int launch_sm100_b(const fa_fwd_params& p, Sm100FwdArgs& a) {
     mark_kernel(st);
     return cuda_ok(cudaGetLastError(), "fwd_sm100 launch");
 }
+// no query block has more than 128 rows
+static bool short_queries(const fa_fwd_params& p, int gq) { return (long)p.sq * gq <= 128; }
 template <typename T, int D>
 static int launch_sm100_t(const fa_fwd_params& p, Sm100FwdArgs& a) {
     const bool bias = p.softcap > 0.f || p.alibi_slopes;
-    // no query block has more than 128 rows
-    if ((long)p.sq * a.gq <= 128) return bias ? launch_sm100_b<T, D, true, true>(p, a) : launch_sm100_b<T, D, false, true>(p, a);
+    if (short_queries(p, a.gq)) return bias ? launch_sm100_b<T, D, true, true>(p, a) : launch_sm100_b<T, D, false, true>(p, a);
     return bias ? launch_sm100_b<T, D, true, false>(p, a) : launch_sm100_b<T, D, false, false>(p, a);
 }
 template <typename T, int D, bool BIAS>
@@ -1124,8 +1125,10 @@ int launch_fwd_sm100(const fa_fwd_params& p, int nsplit, int keys_per_split, flo
         if (p.dtype == FA_F16) return p.d <= 192 ? launch_sm100_wide_t<__half, 192>(p, a) : launch_sm100_wide_t<__half, 256>(p, a);
         return p.d <= 192 ? launch_sm100_wide_t<__nv_bfloat16, 192>(p, a) : launch_sm100_wide_t<__nv_bfloat16, 256>(p, a);
     }
-    note_kernel("sm100_tcgen05_2q");                         // one name for the tcgen05 forward at head dims up to 128
-    if (single_tile(p, a.gq, a.nsplit)) return launch_fwd_single_sm100(p, a);
+    // one name for the tcgen05 forward at head dims up to 128
+    const bool single = single_tile(p, a.gq, a.nsplit);
+    note_kernel("sm100_tcgen05_2q", single ? FORM_ONE_TILE : short_queries(p, a.gq) ? FORM_SHORT_QUERIES : FORM_USUAL);
+    if (single) return launch_fwd_single_sm100(p, a);
     if (p.dtype == FA_F16) return p.d <= 64 ? launch_sm100_t<__half, 64>(p, a) : launch_sm100_t<__half, 128>(p, a);
     return p.d <= 64 ? launch_sm100_t<__nv_bfloat16, 64>(p, a) : launch_sm100_t<__nv_bfloat16, 128>(p, a);
 }

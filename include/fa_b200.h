@@ -311,7 +311,9 @@ void        fa_set_kernel_policy(int policy);
  * timed-out wait in a tcgen05 / TMA kernel (get; synchronises the device), 3 = clear that code (set), 4 = 0 makes
  * the decode kernel load cache tiles with 16-byte cp.async copies instead of TMA (set), 7 = 0 makes the tcgen05
  * backward recompute S and dP in its dQ kernel instead of reading the dS tiles the dK/dV kernel leaves in the
- * workspace (set). */
+ * workspace (set), 8 = which form of the kernel fa_last_kernel() names ran on this thread (get): 0 the usual one,
+ * 1 both softmax groups on the same query rows (at most 128), 2 one query tile a CTA (capped scores), 3 dQ from stored
+ * dS tiles. */
 void        fa_debug_set(int key, int value);
 int         fa_debug_get(int key);
 

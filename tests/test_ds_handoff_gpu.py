@@ -8,10 +8,13 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+STORED_DS = 3                            # fa_debug_get(8): dQ came from stored dS tiles
+
+
 def _compare(run, dt, name):
     import fa_b200_capi as capi
     got = run()
-    assert capi.last_kernel() == name and capi.lib.fa_debug_get(2) == 0
+    assert capi.last_kernel() == name and capi.lib.fa_debug_get(8) == STORED_DS and capi.lib.fa_debug_get(2) == 0
     again = run()
     capi.lib.fa_set_kernel_policy(1)
     try:
@@ -77,7 +80,7 @@ def test_packed_backward_without_room_for_the_tiles(monkeypatch):
     monkeypatch.setattr(capi, "workspace", small)
     b = ext.varlen_bwd(*args)
     torch.cuda.synchronize()
-    assert len(sizes) == 2 and sizes[1] < sizes[0] and capi.lib.fa_debug_get(2) == 0
+    assert len(sizes) == 2 and sizes[1] < sizes[0] and capi.lib.fa_debug_get(8) == 0 and capi.lib.fa_debug_get(2) == 0
     for x, y in zip(a[:3], b[:3]):
         assert (x.float() - y.float()).abs().max().item() <= 2 * 2.0 ** -8 * y.float().abs().max().item()
 

@@ -8,6 +8,8 @@ from parity import assert_lse, assert_within, fwd_refs
 
 pytestmark = pytest.mark.gpu
 
+SHORT_QUERIES = 1                        # fa_debug_get(8): both softmax groups worked on the same rows
+
 # (dtype, B, H, Hkv, Sq, Sk, D, causal, wl, wr, alibi)
 CASES = [
     (torch.bfloat16, 2, 2, 2, 1, 1, 128, False, -1, -1, False),
@@ -33,7 +35,9 @@ def test_short_dense_queries(case):
     out, lse, _ = fa.flash_attn_func(q.cuda(), k.cuda(), v.cuda(), causal=causal, window_size=(wl, wr),
                                      alibi_slopes=None if slopes is None else slopes.cuda(), return_attn_probs=True)
     torch.cuda.synchronize()
+    rows = sq * (h // hkv if sq < 128 else 1)                # a group of heads is stacked into the tile rows
     assert capi.last_kernel() == "sm100_tcgen05_2q" and capi.lib.fa_debug_get(2) == 0
+    assert capi.lib.fa_debug_get(8) == (SHORT_QUERIES if rows <= 128 else 0)
     assert_within("out", out.cpu(), lp_o, f_o)
     assert_lse(lse.cpu(), f_l)
 
@@ -52,6 +56,8 @@ def test_short_packed_queries_and_a_growing_maximum():
     f_o, f_l = orc.attention_varlen_fwd(q.float(), k.float(), v.float(), *cu, 1.0, False, data_type=torch.float32)
     out, lse, _ = fa.flash_attn_varlen_func(q.cuda(), k.cuda(), v.cuda(), cu[0].cuda(), cu[1].cuda(), 128, 700, softmax_scale=1.0,
                                             return_attn_probs=True)
+    import fa_b200_capi as capi
+    assert capi.lib.fa_debug_get(8) == SHORT_QUERIES
     assert_within("out", out.cpu(), lp_o, f_o)
     assert_lse(lse.cpu(), f_l)
 
@@ -76,6 +82,6 @@ def test_short_chunks_against_a_cache(page, sq, h, splits):
     out, lse = fa.flash_attn_with_kvcache(q.cuda(), kc.cuda(), vc.cuda(), cache_seqlens=lens_t.cuda(), causal=True, num_splits=splits,
                                           block_table=None if table is None else table.cuda(), return_softmax_lse=True)
     torch.cuda.synchronize()
-    assert capi.last_kernel() == "sm100_tcgen05_2q" and capi.lib.fa_debug_get(2) == 0
+    assert capi.last_kernel() == "sm100_tcgen05_2q" and capi.lib.fa_debug_get(8) == SHORT_QUERIES and capi.lib.fa_debug_get(2) == 0
     assert_within("out", out.cpu(), lp, f)
     assert_lse(lse.cpu(), fl)

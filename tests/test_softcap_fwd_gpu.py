@@ -8,6 +8,14 @@ from parity import assert_lse, assert_within, fwd_refs
 
 pytestmark = pytest.mark.gpu
 
+ONE_TILE = ("sm100_tcgen05_2q", 2)       # fa_last_kernel(), fa_debug_get(8)
+
+
+def _ran():
+    import fa_b200_capi as capi
+    return capi.last_kernel(), capi.lib.fa_debug_get(8)
+
+
 # (dtype, B, H, Hkv, Sq, Sk, D, causal, wl, wr, cap, spread of q)
 CASES = [
     (torch.bfloat16, 2, 2, 2, 128, 128, 128, False, -1, -1, 30.0, 1.0),
@@ -33,7 +41,7 @@ def test_capped_forward_against_the_oracle(case):
     (lp_o, _), (f_o, f_l) = fwd_refs(q, k, v, scale, causal, (wl, wr), cap)
     out, lse, _ = fa.flash_attn_func(q.cuda(), k.cuda(), v.cuda(), causal=causal, window_size=(wl, wr), softcap=cap, return_attn_probs=True)
     torch.cuda.synchronize()
-    assert capi.lib.fa_debug_get(2) == 0
+    assert capi.lib.fa_debug_get(2) == 0 and _ran() == ONE_TILE
     assert_within("out", out.cpu(), lp_o, f_o)
     assert_lse(lse.cpu(), f_l)
 
@@ -52,6 +60,7 @@ def test_capped_forward_row_maximum_grows_along_the_keys():
     qn[0, 5] = float("nan")
     for x in (q, qn):
         out, lse, _ = fa.flash_attn_func(x.cuda(), k.cuda(), v.cuda(), softmax_scale=1.0, softcap=300.0, return_attn_probs=True)
+        assert _ran() == ONE_TILE
         keep = torch.arange(130) != 5 if x is qn else slice(None)
         assert_within("out", out.cpu()[:, keep], lp_o[:, keep], f_o[:, keep])
         assert_lse(lse.cpu()[..., keep], f_l[..., keep])
@@ -79,6 +88,6 @@ def test_capped_prefill_against_a_cache(page, sq, splits):
                                           block_table=None if table is None else table.cuda(), causal=True, softcap=cap, num_splits=splits,
                                           return_softmax_lse=True)
     torch.cuda.synchronize()
-    assert capi.lib.fa_debug_get(2) == 0
+    assert capi.lib.fa_debug_get(2) == 0 and _ran() == ONE_TILE
     assert_within("out", out.cpu(), lp, f)
     assert_lse(lse.cpu(), fl)
