@@ -308,3 +308,21 @@ def require_cuda(*tensors):
 
 def workspace(nbytes, device):
     return torch.empty(max(int(nbytes), 16), dtype=torch.uint8, device=device)
+
+
+_LARGE_WORKSPACE = 256 << 20
+
+
+def workspace_fits(nbytes, device):
+    """Whether a large workspace can be had at all: not when it exceeds what the caching allocator holds unused and the device
+    has free together.  Trying regardless would make the allocator give all it holds back to the driver before it reports the
+    failure, in every call of a loop whose workspace never fits.  Asking costs 8 us, and 75 when the driver has to be asked
+    too, beside the 150 or more that kernels with such a workspace run."""
+    if nbytes < _LARGE_WORKSPACE or torch.cuda.is_current_stream_capturing():
+        return True
+    stats = torch.cuda.memory.memory_stats_as_nested_dict(device)
+    try:
+        held = stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"]
+    except KeyError:                                         # an allocator that keeps no such counts
+        return True
+    return nbytes <= held or nbytes <= held + torch.cuda.mem_get_info(device)[0]

@@ -357,9 +357,10 @@ def _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p
         *leaves, softmax_lse.data_ptr(), *lse_strides, *cu, batch, sq, sk, total_q, total_k, hq, hkv, q.size(-1), v.size(-1),
         softmax_scale, softcap, int(is_causal), _i32(wl), _i32(wr), _dtype_code(q), int(deterministic), 0, 0,
         capi.raw_stream(device), alibi, alibi_sb)
-    try:
-        ws = capi.workspace(capi._bwd_bytes(buf), device)
-    except torch.OutOfMemoryError:                           # without room for P and dS tiles the kernels recompute them
+    nbytes = capi._bwd_bytes(buf)
+    try:                                                     # without room for P and dS tiles the kernels recompute them
+        ws = capi.workspace(nbytes if capi.workspace_fits(nbytes, device) else capi._bwd_min_bytes(buf), device)
+    except torch.OutOfMemoryError:
         ws = capi.workspace(capi._bwd_min_bytes(buf), device)
     capi.set_workspace(capi.BWD_BLOCK, buf, ws, ws.numel())
     capi.launch(capi._call_varlen_bwd if packed else capi._call_bwd, buf, device)
