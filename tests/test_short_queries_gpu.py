@@ -37,7 +37,7 @@ def test_short_dense_queries(case):
     torch.cuda.synchronize()
     rows = sq * (h // hkv if sq < 128 else 1)                # a group of heads is stacked into the tile rows
     assert capi.last_kernel() == "sm100_tcgen05_2q" and capi.lib.fa_debug_get(2) == 0
-    assert capi.lib.fa_debug_get(8) == (SHORT_QUERIES if rows <= 128 else 0)
+    assert capi.lib.fa_debug_get(8) == (SHORT_QUERIES if rows <= 128 and sk > 128 else 0)      # one key tile is not shared out
     assert_within("out", out.cpu(), lp_o, f_o)
     assert_lse(lse.cpu(), f_l)
 
