@@ -71,27 +71,38 @@ static int check_common(const fa_fwd_params& p) {
     return FA_OK;
 }
 
-// Key splits of a prefill chunk: none, as many as one wave of CTAs holds, or `most` (about two waves).  The lengths are not known here, so each count is rated by the mean of two
-// estimates in microseconds, every sequence as long as the capacity (whole waves of CTAs) and lengths spread below it (0.6
-// of the keys, and the longest sequence at least); both with what a split costs, 6 us to start and finish a CTA and the
-// partials' way to memory and back.  A larger count has to be rated 5 % better.  Measured, 512 new tokens, H32/8 D128: B4
-// up to 16000 keys 238 us unsplit, 278 with two splits (which two waves of CTAs asked for); B1 16000 keys 224 / 138 / 153
-// us with one / two / four; B6 S300 H16 up to 32000 keys 542 / 428 with one / two.  Counts between one wave and `most` are
-// not tried: a second wave that is mostly empty made them the worst (B4 S128 up to 30000 keys: 150 / 160 / 132 us with one /
-// two / three).
+// Key splits of a prefill chunk: none, as many as one wave of CTAs holds, or `most` (about two waves, or 2048 keys a split).
+// The lengths are not known here, so each count is rated by the mean of two estimates in microseconds, every sequence as
+// long as the capacity (whole waves of CTAs) and lengths spread below it (0.6 of the keys, and the longest sequence at
+// least); both with what a split costs, 6 us to start and finish a CTA and the partials' way to memory and back.  A larger
+// count has to be rated 5 % better.  The tile times are those of head dim 128; head dim 64 takes 0.86 of them and rates
+// the same counts.  Counts in between are not tried: a second wave that is mostly empty makes them the worst, and below
+// one wave more splits are better.
+// Measured at head dims 64 and 128 on 234 shapes (B1-8, 64-2048 new tokens, capacities 4096-32768) against `most`: 7 % faster
+// in the geometric mean; 12-28 % where the lengths are near the capacity and one wave holds two to four splits (B1 of 512
+// tokens, H32/8 D128, 11264 keys: 129 -> 93 us), 17 to 32 % where the chunk is better left unsplit (B4 S512 H32/8 D128 up to
+// 13312 keys, B1 S1024 of 5120).  What it costs: two
+// sequences of which one is half as long, 32 or 64 CTAs a split, up to 22 % (B2 S256 H16 D64, 11205 and 5185 keys: 42 -> 51
+// us), because the splits past the shorter one's end leave room for a second wave; more CTAs than SMs with query blocks of
+// uneven size and uneven lengths, up to 10 % (B8 S300 H16/4 D128 up to 7680 keys: 173 -> 182 us; with even lengths up to 4096
+// it is 156 -> 137).
+// Capped scores have a kernel that keeps two CTAs an SM: with more CTAs than SMs they stay split (B4 S512 H32/8 up to 32768
+// keys, cap 30: 1108 us split, 1257 unsplit at D64; 1429 / 1598 at D128).
 static int prefill_splits(const fa_fwd_params& p, long ctas, int most) {
-    const double sms = sm_count(), tiles = (p.sk + 127) / 128;
-    const double whole = tiles * (ctas * 256 <= (long)p.b * p.sq * p.hq * 2 ? 1.9 : 1.0);        // a CTA over all keys: two query tiles or one
-    const double rows = (double)p.b * p.sq * p.hq;
+    const long sms = sm_count();
+    const double rows = (double)p.b * p.sq * p.hq, tiles = (p.sk + 127) / 128;
+    if (ctas > sms && p.softcap > 0.f) return most;
+    const double whole = tiles * (ctas * 256 <= rows * 2 ? 1.9 : 1.0);           // a CTA over all keys: two query tiles or one
+    const long wave = sms / ctas < 1 ? 1 : sms / ctas;
+    const int counts[3] = {1, (int)(wave < most ? wave : most), most};
     int best = 1;
     double best_us = 0;
-    for (int n = 1; n <= most; ++n) {
-        if (n > 1 && n < most && ctas * n > (long)sms) continue;
-        const double one = whole / n, waves = (double)((long)((ctas * n + (long)sms - 1) / (long)sms));
+    for (int n : counts) {
+        const double one = whole / n, waves = (double)((ctas * n + sms - 1) / sms);
         const double spread = 0.6 * ctas * whole / sms + 0.25 * one;
-        const double cost = ctas * n / sms * 6.0 + (n > 1 ? rows * p.d * 8.0 * n / 4e6 + 5.0 : 0.0);
+        const double cost = ctas * n * 6.0 / sms + (n > 1 ? rows * p.d * 8.0 * n / 4e6 + 5.0 : 0.0);
         const double us = 0.5 * (waves * one + (spread > one ? spread : one)) + cost;
-        if (n == 1 || us < 0.95 * best_us) { best = n; best_us = us; }
+        if (best_us == 0 || us < 0.95 * best_us) { best = n; best_us = us; }
     }
     return best;
 }
