@@ -237,7 +237,9 @@ __global__ void __launch_bounds__(608, 1) bwd_wide_scores_kernel(const __grid_co
             tmem_ld32(tmem + lane_base + COL_S + buf * 128 + cg * 32, pr);
             tmem_wait_ld();
             const bool inside = __all_sync(0xffffffffu, i0 >= qi_lo && i0 + 31 <= qi_hi);
-            auto seen = [&](int i) { return i0 + i >= qi_lo && i0 + i <= qi_hi; };
+            // a packed sequence ends inside the tile: how many of the thread's 32 columns are its own
+            const bool past_end = a.cu_q && (n0 + 128 > sk || (m + 1) * 128 > sq);
+            const int own = n < sk ? sq - i0 : 0;
             float slope = 0.f;
             if constexpr (BIAS) { if (a.alibi) slope = a.alibi[(int64_t)b * a.alibi_sb + hk * G + g] * kLog2e; }
 #pragma unroll
@@ -270,8 +272,11 @@ __global__ void __launch_bounds__(608, 1) bwd_wide_scores_kernel(const __grid_co
                 float2 p01 = make_float2(ex2_approx(x01.x), ex2_approx(x01.y));
                 float2 p23 = make_float2(ex2_approx(x23.x), ex2_approx(x23.y));
                 if (!inside) {
-                    p01 = make_float2(seen(i) ? p01.x : 0.f, seen(i + 1) ? p01.y : 0.f);
-                    p23 = make_float2(seen(i + 2) ? p23.x : 0.f, seen(i + 3) ? p23.y : 0.f);
+                    const int qi = i0 + i;
+                    p01.x = (qi >= qi_lo && qi <= qi_hi) ? p01.x : 0.f;
+                    p01.y = (qi + 1 >= qi_lo && qi + 1 <= qi_hi) ? p01.y : 0.f;
+                    p23.x = (qi + 2 >= qi_lo && qi + 2 <= qi_hi) ? p23.x : 0.f;
+                    p23.y = (qi + 3 >= qi_lo && qi + 3 <= qi_hi) ? p23.y : 0.f;
                 }
                 pr[i] = __float_as_uint(p01.x * fac[0]); pr[i + 1] = __float_as_uint(p01.y * fac[1]);
                 pr[i + 2] = __float_as_uint(p23.x * fac[2]); pr[i + 3] = __float_as_uint(p23.y * fac[3]);
@@ -295,11 +300,11 @@ __global__ void __launch_bounds__(608, 1) bwd_wide_scores_kernel(const __grid_co
                                         add2(make_float2(__uint_as_float(dr[i]), __uint_as_float(dr[i + 1])), make_float2(nd.x, nd.y)));
                 float2 d23 = mul2(make_float2(__uint_as_float(pr[i + 2]), __uint_as_float(pr[i + 3])),
                                         add2(make_float2(__uint_as_float(dr[i + 2]), __uint_as_float(dr[i + 3])), make_float2(nd.z, nd.w)));
-                if (!inside) {
+                if (past_end) {
                     // selected, not multiplied: the rows that a tile copy fetched past the end of a packed sequence are its
                     // neighbour's, and 0 x NaN is NaN
-                    d01 = make_float2(seen(i) ? d01.x : 0.f, seen(i + 1) ? d01.y : 0.f);
-                    d23 = make_float2(seen(i + 2) ? d23.x : 0.f, seen(i + 3) ? d23.y : 0.f);
+                    d01 = make_float2(i < own ? d01.x : 0.f, i + 1 < own ? d01.y : 0.f);
+                    d23 = make_float2(i + 2 < own ? d23.x : 0.f, i + 3 < own ? d23.y : 0.f);
                 }
                 w[i / 2] = Elem<T>::pack(d01.x, d01.y);
                 w[i / 2 + 1] = Elem<T>::pack(d23.x, d23.y);
@@ -422,6 +427,9 @@ __global__ void __launch_bounds__(192, 1) bwd_wide_grads_kernel(const __grid_con
             }
         }
     } else if (warp == 1) {
+        // the block in which a packed sequence ends, if it ends inside one
+        const int b_rows = is_q ? sk : sq, tail = a.cu_q && (b_rows & 127) ? b_rows >> 7 : -1;
+        int other = br.lo;
         bool ok = true;
         for (int j = 0; j < steps && ok; ++j) {
             const int st = j & 1;
@@ -429,30 +437,33 @@ __global__ void __launch_bounds__(192, 1) bwd_wide_grads_kernel(const __grid_con
             if (!ok) break;
             tc_fence_after();
             const uint32_t s0 = sbase + st * L::kStage;
-            if (a.cu_q) {
-                // rows past the end of a packed sequence are the next one's and meet zeros of the tile: cleared, so that a NaN
-                // or infinity stays in its own sequence (past the end of a dense batch entry the copy fills with zeros)
-                const int other = br.lo + (is_q ? j : j % (br.hi - br.lo));
-                const int first = (is_q ? sk : sq) - other * 128;
-                if (first < 128) {
-#pragma unroll
-                    for (int sub = 0; sub < NSUB; ++sub)
-                        for (int idx = first * 8 + lane; idx < 128 * 8; idx += 32)          // 16-byte chunks of rows first .. 127
-                            *reinterpret_cast<uint4*>(sgen + st * L::kStage + kWideTileBytes + sub * kSub + idx * 16) = make_uint4(0, 0, 0, 0);
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                }
-            }
             const uint64_t dB = umma_desc(s0 + (uint32_t)kWideTileBytes, kSub, 1024);
             // Stored tile: element (key k, query q) at chunk (q / 8) x 2048 + k x 16 + (q % 8) x 2 bytes.
-            if (!is_q) {
-                // K step = 16 queries = 2 chunks; along K the chunks lie 2048 bytes apart, along M eight keys are 128 bytes
-                const uint64_t dA = umma_desc_noswizzle(s0, 2048, 128);
+            // dV, dK: a K step is 16 queries = 2 chunks; along K the chunks lie 2048 bytes apart, along M eight keys are 128
+            // bytes.  dQ: a K step is 16 keys = 256 bytes; along K eight keys are 128 bytes, along M the chunks lie 2048 apart.
+            const uint64_t dA = is_q ? umma_desc_noswizzle(s0, 128, 2048) : umma_desc_noswizzle(s0, 2048, 128);
+            const int block = other;                         // query block (dV, dK) or key block (dQ)
+            if (++other == br.hi) other = br.lo;
+            if (block == tail) {
+                // Rows past the end of a packed sequence are the next one's and meet zeros of the tile, but 0 x NaN is NaN (past
+                // the end of a dense batch entry the copy fills with zeros): only the K steps that hold own rows are multiplied,
+                // and what is left of the last one is cleared.
+                const int left = b_rows & 127, end = (left + 15) & ~15;
+#pragma unroll
+                for (int sub = 0; sub < NSUB; ++sub)
+                    for (int idx = left * 8 + lane; idx < end * 8; idx += 32)       // 16-byte chunks of rows left .. end - 1
+                        *reinterpret_cast<uint4*>(sgen + st * L::kStage + kWideTileBytes + sub * kSub + idx * 16) = make_uint4(0, 0, 0, 0);
+                fence_proxy_async_smem();
+                __syncwarp();
+                for (int k = 0; k < end; k += 16) {
+                    const uint64_t ak = umma_desc_at(dA, k * (is_q ? 16 : 256)), bk = umma_desc_at(dB, k * 128);
+                    if (j == 0 && k == 0) umma_ss_w<0>(tmem, ak, bk, is_q ? IDESC_Q : IDESC_KV);
+                    else umma_ss_w<1>(tmem, ak, bk, is_q ? IDESC_Q : IDESC_KV);
+                }
+            } else if (!is_q) {
                 umma_ss_group4<0, 256, 512, 768, 0, 128, 256, 384>(tmem, dA, dB, IDESC_KV, j > 0);
                 umma_ss_group4<1024, 1280, 1536, 1792, 512, 640, 768, 896>(tmem, dA, dB, IDESC_KV, 1);
             } else {
-                // K step = 16 keys = 256 bytes; along K eight keys are 128 bytes, along M the chunks lie 2048 bytes apart
-                const uint64_t dA = umma_desc_noswizzle(s0, 128, 2048);
                 umma_ss_group4<0, 16, 32, 48, 0, 128, 256, 384>(tmem, dA, dB, IDESC_Q, j > 0);
                 umma_ss_group4<64, 80, 96, 112, 512, 640, 768, 896>(tmem, dA, dB, IDESC_Q, 1);
             }
