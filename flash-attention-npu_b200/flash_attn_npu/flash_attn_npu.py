@@ -318,14 +318,18 @@ def _bwd_common(dout, q, k, v, out, softmax_lse, dq_, dk_, dv_, alibi_slopes_, p
     dq = torch.empty_like(q) if dq_ is None else dq_
     dk = torch.empty_like(k) if dk_ is None else dk_
     dv = torch.empty_like(v) if dv_ is None else dv_
+    # The caller of a backward does not choose how autograd lays out the gradient of the output (a slice of a concatenation):
+    # what 16-byte loads cannot read in place is copied.  So are expanded inputs (the gradient of a sum, keys shared by heads),
+    # which tile copies cannot read.
+    s = dout.stride()
+    if s[-1] == 1 and (dout.data_ptr() % 16 or (s[0] | s[1] | s[-2]) % 8):
+        dout = dout.clone(memory_format=torch.contiguous_format)
     leaves, copies = [], []
-    for i, t in enumerate((dout, q, k, v, out, dq, dk, dv)):
+    for t in (dout, q, k, v, out, dq, dk, dv):
         s = t.stride()
         if s[-1] != 1:
             raise RuntimeError("Input tensor must have contiguous last dimension")
-        if i < 5 and (t.data_ptr() % 16 or min(s) <= 0 or (s[0] | s[1] | s[-2]) % 8):
-            # The caller of a backward does not choose how autograd lays out the gradient of the output (a slice of a
-            # concatenation, an expanded sum): what the 16-byte loads and tile copies cannot read in place is copied.
+        if 0 in s and len(leaves) < 20:                      # one of the five inputs
             t = t.clone(memory_format=torch.contiguous_format)
             copies.append(t)
             s = t.stride()

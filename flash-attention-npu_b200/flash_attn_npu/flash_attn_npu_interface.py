@@ -201,7 +201,7 @@ def _dense_backward(ctx, dout, dq=None, dk=None, dv=None):
     else:
         views = True
     if (_scalars_ok(ctx.dropout_p, ctx.softmax_scale, ctx.causal, ctx.window_size, ctx.softcap) and type(ctx.deterministic) is bool
-            and _plain(dout, q, k, v, out, lse, dq, dk, dv, ctx.alibi_slopes)):
+            and _plain(dout, q, k, v, out, lse, ctx.alibi_slopes)):
         _ext._bwd_common(maybe_contiguous(dout), maybe_contiguous(q), maybe_contiguous(k), maybe_contiguous(v), maybe_contiguous(out),
                          lse, dq, dk, dv, ctx.alibi_slopes, ctx.dropout_p, ctx.softmax_scale, ctx.causal, ctx.window_size[0],
                          ctx.window_size[1], ctx.softcap, ctx.deterministic)
@@ -242,7 +242,7 @@ def _varlen_backward(ctx, dout):
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
     if (_scalars_ok(ctx.dropout_p, ctx.softmax_scale, ctx.causal, ctx.window_size, ctx.softcap) and type(ctx.deterministic) is bool
             and type(ctx.max_seqlen_q) is int and type(ctx.max_seqlen_k) is int
-            and _plain(dout, q, k, v, out, lse, dq, dk, dv, cu_q, cu_k, ctx.alibi_slopes)):
+            and _plain(dout, q, k, v, out, lse, cu_q, cu_k, ctx.alibi_slopes)):
         _ext._bwd_common(maybe_contiguous(dout), maybe_contiguous(q), maybe_contiguous(k), maybe_contiguous(v), maybe_contiguous(out),
                          lse, dq, dk, dv, ctx.alibi_slopes, ctx.dropout_p, ctx.softmax_scale, ctx.causal, ctx.window_size[0],
                          ctx.window_size[1], ctx.softcap, ctx.deterministic, cu_q, cu_k, ctx.max_seqlen_q, ctx.max_seqlen_k)

@@ -167,7 +167,7 @@ def _run_backward(ctx, dout, q, k, v, out, lse, cu_q=None, cu_k=None, max_q=None
     assert ctx.attention_chunk == 0, "backward does not support attention_chunk"
     dout, q, k, v, out, og = _pad_bwd_headdim(dout, q, k, v, out)
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    if _direct((dout, q, k, v, out, lse, cu_q, cu_k, dq, dk, dv), (ctx.softmax_scale, ctx.softcap),
+    if _direct((dout, q, k, v, out, lse, cu_q, cu_k), (ctx.softmax_scale, ctx.softcap),
                (ctx.window_size[0], ctx.window_size[1], ctx.sm_margin), (max_q, max_k), (ctx.causal, ctx.deterministic)):
         _v2_ext._bwd_common(*[maybe_contiguous(x) for x in (dout, q, k, v, out)], lse, dq, dk, dv, None, 0.0, ctx.softmax_scale,
                             ctx.causal, ctx.window_size[0], ctx.window_size[1], ctx.softcap, ctx.deterministic, cu_q, cu_k, max_q, max_k)
