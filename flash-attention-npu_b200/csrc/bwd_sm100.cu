@@ -990,7 +990,8 @@ int launch_bwd_sm100(const fa_bwd_params& p) {
     a.lse = p.lse; a.lse_sb = p.lse_stride_b; a.lse_sh = p.lse_stride_h; a.lse_ss = p.lse_stride_s;
     a.delta = reinterpret_cast<const float*>(p.workspace);
     a.ds_tiles = nullptr; a.nkb = (p.sk + 127) / 128; a.nqb = (p.sq + 127) / 128;
-    if (g_ds_spill && ds_tiles_bytes(p) > 0 && p.workspace_bytes >= delta_bytes(p) + ds_tiles_bytes(p)) {
+    // bulk copies read the tiles: 16-byte aligned, or recomputed
+    if (g_ds_spill && ds_tiles_bytes(p) > 0 && p.workspace_bytes >= delta_bytes(p) + ds_tiles_bytes(p) && reinterpret_cast<uintptr_t>(p.workspace) % 16 == 0) {
         a.ds_tiles = reinterpret_cast<unsigned char*>(p.workspace) + delta_bytes(p);
     }
     a.cu_q = p.cu_seqlens_q; a.cu_k = p.cu_seqlens_k;

@@ -313,8 +313,9 @@ static int run_backward(const fa_bwd_params& pin) {
     if (!p.workspace || p.workspace_bytes < need)
         return fail(FA_ERR_WORKSPACE, "workspace of %zu bytes required, %zu given", need, p.workspace_bytes);
     if (fast) return launch_bwd_sm100(p);
-    // above head dim 128 the tcgen05 kernels need room for P and dS tiles (up to 6 GiB); without it the general kernels run
-    const bool wide = g_policy == 0 && bwd_wide_sm100_supported(p) && p.workspace_bytes >= bwd_wide_sm100_workspace(p);
+    // above head dim 128 the tcgen05 kernels need room for P and dS tiles (up to 6 GiB), 16-byte aligned for their bulk copies;
+    // without it the general kernels run
+    const bool wide = g_policy == 0 && bwd_wide_sm100_supported(p) && aligned16(p.workspace) && p.workspace_bytes >= bwd_wide_sm100_workspace(p);
     return wide ? launch_bwd_wide_sm100(p) : launch_bwd_generic(p);
 }
 

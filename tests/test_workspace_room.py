@@ -45,3 +45,27 @@ def test_backward_does_not_try_what_cannot_fit(d, kernel, monkeypatch):
     assert capi.last_kernel() == kernel and len(sizes) == 1 and sizes[0] < 1 << 20 and capi.lib.fa_debug_get(2) == 0
     for x, y in zip(got, want):                              # roundings of P, dS and the result
         assert (x.float() - y.float()).abs().max().item() <= 3 * 2.0 ** -8 * y.float().abs().max().item()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d,packed,kernel", [(128, False, "sm100_tcgen05_bwd"), (128, True, "sm100_tcgen05_bwd"), (256, False, "generic_mma_bwd"), (192, True, "generic_mma_bwd")])
+def test_a_workspace_aligned_for_floats_only_holds_no_tiles(d, packed, kernel, monkeypatch):
+    """Bulk copies want 16-byte addresses; a C caller's workspace may start on any float."""
+    from flash_attn_npu import flash_attn_npu as ext
+    s, h = 300, 4
+    q, k, v, do = (torch.randn(*((2 * s, h, d) if packed else (2, s, h, d)), device="cuda").bfloat16() for _ in range(4))
+    cu = torch.tensor([0, s, 2 * s], dtype=torch.int32, device="cuda")
+    if packed:
+        out, lse, _, _ = ext.varlen_fwd(q, k, v, None, cu, cu, None, None, None, None, s, s, 0.0, 0.1, False, True, -1, -1, 0.0, False, None)
+        run = lambda: ext.varlen_bwd(do, q, k, v, out, lse, None, None, None, cu, cu, None, s, s, 0.0, 0.1, False, True, -1, -1, 0.0, False, None, None)[:3]  # noqa: E731
+    else:
+        out, lse, _, _ = ext.fwd(q, k, v, None, None, 0.0, 0.1, True, -1, -1, 0.0, False, None)
+        run = lambda: ext.bwd(do, q, k, v, out, lse, None, None, None, None, 0.0, 0.1, True, -1, -1, 0.0, False, None, None)[:3]  # noqa: E731
+    want = run()
+    real = capi.workspace
+    monkeypatch.setattr(capi, "workspace", lambda n, device: real(n + 16, device)[4:4 + n])
+    got = run()
+    torch.cuda.synchronize()
+    assert capi.last_kernel() == kernel and capi.lib.fa_debug_get(8) == 0 and capi.lib.fa_debug_get(2) == 0
+    for x, y in zip(got, want):                              # roundings of P, dS and the result
+        assert (x.float() - y.float()).abs().max().item() <= 3 * 2.0 ** -8 * y.float().abs().max().item()
