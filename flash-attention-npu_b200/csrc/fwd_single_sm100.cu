@@ -350,7 +350,9 @@ __global__ void __launch_bounds__(320, 2) fwd_single_sm100_kernel(const __grid_c
                 }
             }
             float m_loc = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-            m_loc = m_loc == -INFINITY ? m_loc : cap_out * tanh_any(m_loc * cap_in2);      // the cap is monotone; log2 domain
+            // the cap is monotone; log2 domain.  It makes a finite score of an infinite one, so that -inf only stands for a row
+            // that sees none of these keys.
+            m_loc = klo <= khi && klo <= n0 + 63 && khi >= n0 ? cap_out * tanh_any(m_loc * cap_in2) : -INFINITY;
             // one of the 64 threads moves its base (or gave up waiting): both warps take the slow way
             if (pair_any(bid, !ok || m_loc > m_used + kRescaleThreshold)) {
                 s_max[half * 128 + r] = m_loc;

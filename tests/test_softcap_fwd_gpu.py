@@ -91,3 +91,25 @@ def test_capped_prefill_against_a_cache(page, sq, splits):
     assert capi.lib.fa_debug_get(2) == 0 and _ran() == ONE_TILE
     assert_within("out", out.cpu(), lp, f)
     assert_lse(lse.cpu(), fl)
+
+
+@pytest.mark.parametrize("sign", [-1.0, 1.0])
+@pytest.mark.parametrize("d,causal,win", [(64, False, (-1, -1)), (128, True, (-1, -1)), (128, True, (90, 0))])
+def test_infinite_scores_are_capped(d, causal, win, sign):
+    """The cap makes a finite score of an infinite one: such a row averages the values it sees, and its LSE is sign * cap + ln(keys)."""
+    import math
+    import fa_b200_capi as capi
+    import flash_attn_npu as fa
+    b, s, h, cap = 1, 300, 2, 200.0
+    q, k, v = (torch.randn(b, s, h, d) for _ in range(3))
+    q[:, ::3], k[..., 1:], k[..., 0] = 0.0, 0.0, 1.0
+    q[:, ::3, :, 0] = sign * math.inf
+    q, k, v = (t.bfloat16() for t in (q, k, v))
+    out, lse, _ = fa.flash_attn_func(q.cuda(), k.cuda(), v.cuda(), causal=causal, window_size=win, softcap=cap, return_attn_probs=True)
+    torch.cuda.synchronize()
+    assert capi.lib.fa_debug_get(2) == 0 and _ran() == ONE_TILE
+    for i in range(0, s, 3):
+        lo, hi = (max(0, i - win[0]) if win[0] >= 0 else 0), (i if causal else s - 1)
+        want = v[:, lo:hi + 1].float().mean(1)
+        assert (out[:, i].cpu().float() - want).abs().max() <= 2.0 ** -7 * max(1.0, want.abs().max().item()), i
+        assert (lse[..., i].cpu() - (sign * cap + math.log(hi - lo + 1))).abs().max() <= 1e-3, i
