@@ -220,9 +220,12 @@ else:
         return torch.cuda.current_stream(device).cuda_stream
 
 
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+
+
 def launch(fn, buf, device):
     """Run an entry point with `device` current."""
-    if torch.cuda.current_device() == device.index:
+    if _current_device() == device.index:
         check(fn(buf))
     else:
         with torch.cuda.device(device):
