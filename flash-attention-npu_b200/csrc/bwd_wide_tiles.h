@@ -38,16 +38,23 @@ FA_HD BlockRange wide_query_blocks(const WideGrid& t, int sq, int sk, int n) {
     return r;
 }
 
-// key blocks that reach query block m: they form one range
+// key blocks that reach query block m: the n for which wide_query_blocks holds m, one range
 FA_HD BlockRange wide_key_blocks(const WideGrid& t, int sq, int sk, int m) {
+    const int diff = sk - sq, wr = t.causal ? 0 : t.wr;
+    const int blocks = (sk + 127) / 128 < t.nkb ? (sk + 127) / 128 : t.nkb;
+    const int last = m * 128 + 127 < sq - 1 ? m * 128 + 127 : sq - 1;                // last row of the block
     BlockRange r;
-    r.lo = t.nkb;
-    r.hi = 0;
-    for (int n = 0; n < t.nkb && n * 128 < sk; ++n) {
-        const BlockRange q = wide_query_blocks(t, sq, sk, n);
-        if (m < q.lo || m >= q.hi) continue;
-        if (n < r.lo) r.lo = n;
-        r.hi = n + 1;
+    r.lo = 0;
+    r.hi = m < t.nqb && m * 128 < sq ? blocks : 0;
+    if (wr >= 0) {                                           // the block's first key is at most wr past some row's diagonal
+        const int key = last + diff + wr;
+        const int hi = key < 0 ? 0 : key / 128 + 1;
+        if (hi < r.hi) r.hi = hi;
+    }
+    if (t.wl >= 0) {                                         // the block's last key is at most wl before the first row's diagonal
+        const int key = m * 128 + diff - t.wl;
+        if (key > sk - 1) r.hi = 0;
+        else if (key > 0) r.lo = key / 128;
     }
     return r;
 }
