@@ -85,8 +85,6 @@ def test_both_routes_give_the_same_bits(version, packed, d, monkeypatch):
     from flash_attn_npu_3 import flash_attn_npu_interface as i3
     fa = fa2 if version == 2 else fa3
     q, k, v, do = _inputs(d=d)
-    if version == 3 and d == 100:
-        pytest.skip("the v3 backward wants a multiple of 8, as before")
     cu = torch.tensor([0, 130, 260], dtype=torch.int32, device="cuda")
 
     def step(softcap):

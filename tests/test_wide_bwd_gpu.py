@@ -183,3 +183,26 @@ def test_capped_scores_keep_their_precision(cap):
     assert capi.last_kernel() == "sm100_wide_tcgen05_bwd"
     for n, g, a, r in zip(("dq", "dk", "dv"), got, lp, f32):
         assert_within(n, g.cpu(), a, r, roundings=3)
+
+
+@pytest.mark.parametrize("dt,d,causal,win,cap", [
+    (torch.float16, 256, False, (60, 30), 0.0), (torch.bfloat16, 192, True, (100, 0), 0.0), (torch.float16, 160, True, (-1, -1), 4.0),
+    (torch.bfloat16, 256, False, (-1, -1), 0.0), (torch.float16, 248, False, (0, 150), 2.0)])
+def test_wide_packed_backward_with_windows_and_caps(dt, d, causal, win, cap):
+    import fa_b200_capi as capi
+    from flash_attn_npu import flash_attn_npu as ext
+    lq, lk, h, hkv = [300, 0, 129, 64, 1], [260, 70, 400, 1, 130], 4, 2
+    q, do = ((torch.rand(sum(lq), h, d) * 2 - 1).to(dt) for _ in range(2))
+    k, v = ((torch.rand(sum(lk), hkv, d) * 2 - 1).to(dt) for _ in range(2))
+    cu = [torch.tensor([0] + torch.tensor(x).cumsum(0).tolist(), dtype=torch.int32) for x in (lq, lk)]
+    scale = d ** -0.5
+    out, lse = orc.attention_varlen_fwd(q.float(), k.float(), v.float(), *cu, scale, causal, win, cap, data_type=torch.float32)
+    lp = orc.attention_varlen_bwd(q, k, v, do, lse, *cu, scale, causal, win, cap)
+    f32 = orc.attention_varlen_bwd(q.float(), k.float(), v.float(), do.float(), lse, *cu, scale, causal, win, cap)
+    qg, kg, vg, dog, og, lg, cq, ck = (t.cuda() for t in (q, k, v, do, out.to(dt), lse, *cu))
+    g = [torch.full_like(t, 777.0) for t in (qg, kg, vg)]
+    ext.varlen_bwd(dog, qg, kg, vg, og, lg, *g, cq, ck, None, max(lq), max(lk), 0.0, scale, False, causal, *win, cap, False, None, None)
+    torch.cuda.synchronize()
+    assert capi.last_kernel() == "sm100_wide_tcgen05_bwd" and capi.lib.fa_debug_get(2) == 0
+    for n, x, a, r in zip(("dq", "dk", "dv"), g, lp, f32):
+        assert_within(n, x.cpu(), a, r, roundings=3)
