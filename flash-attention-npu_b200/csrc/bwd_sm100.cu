@@ -890,7 +890,7 @@ int launch_bwd_delta_sm100(const fa_bwd_params& p, float* delta) {
     return cuda_ok(cudaGetLastError(), "bwd_delta launch");
 }
 
-// 1 (default): dense calls hand dS^T from the dK/dV kernel to a one-GEMM dQ kernel through the workspace;
+// 1 (default): calls within the workspace limit hand dS^T from the dK/dV kernel to a one-GEMM dQ kernel through the workspace;
 // 0: the dQ kernel always recomputes S and dP (fa_debug_set key 7)
 static std::atomic<int> g_ds_spill{1};
 void bwd_sm100_set_ds_spill(int v) { g_ds_spill = v; }

@@ -497,7 +497,9 @@ __global__ void __launch_bounds__(192, 1) bwd_wide_grads_kernel(const __grid_con
 // Tiles of the KV heads of one launch: what a launch writes should still be in the 126 MB L2 when the next launch reads
 // it, and one launch should fill the GPU.  Under a causal mask about half of a head's tiles exist.  Measured at
 // B2 S2048 H8/4 / B1 S8192 H8 / B4 S1024 H16 (causal) with 32, 64, 128 MiB: 223 / 151 / 133, 1147 / 1050 / 1002,
-// 238 / 212 / 211 us.
+// 238 / 212 / 211 us.  A KV head whose tiles alone are more than L2 goes by itself, through HBM, at about the same rate: whole
+// training steps at D256 causal B1 S8192, H8 on one KV head (2 GiB of tiles) 1150 us, on eight (256 MiB each) 1295; D192
+// full B1 S12000 H8 on one, 3730 us = 830 TFLOP/s.
 constexpr size_t kWideGroupBytes = (size_t)128 << 20;
 constexpr size_t kWideWorkspaceLimit = (size_t)6 << 30;      // one KV head's tiles may take this much at most
 

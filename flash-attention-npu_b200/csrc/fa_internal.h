@@ -79,7 +79,7 @@ bool bwd_wide_sm100_supported(const fa_bwd_params& p);
 size_t bwd_wide_sm100_workspace(const fa_bwd_params& p);
 int launch_bwd_wide_sm100(const fa_bwd_params& p);
 int bwd_wide_error_flag(bool clear);
-// 1 (default): dense calls hand dS^T tiles from the dK/dV kernel to a one-GEMM dQ kernel (fa_debug_set key 7)
+// 1 (default): calls within the workspace limit hand dS^T tiles from the dK/dV kernel to a one-GEMM dQ kernel (fa_debug_set key 7)
 void bwd_sm100_set_ds_spill(int v);
 // true while the caller has lent per-kernel timing events to this thread
 bool kernel_events_active();

@@ -49,7 +49,8 @@ struct FwdSm100Smem2 {
 // Pairs of every 8 whose exponential runs on the FMA pipe.  The special-function unit is not the limiter and the
 // polynomial costs six times the instructions, so a few are enough.  Head dim 128: 1 of 8 against 2 and 0, packed causal
 // prefill of the benchmark under the power cap 3841 / 3916 / 3869 us.  Head dim 64, full attention B1 S8192 H37: 814 us with
-// 2, 859 with 1, 858 with 3.
+// 2, 859 with 1, 858 with 3.  Head dims 192 and 256 run with the 2 they were written with; other shares are not measured
+// there.
 template <int D> constexpr int kFwdPoly = D == 128 ? 1 : 2;
 enum { C_Q = 0, C_KF0, C_KF1, C_KF2, C_KE0, C_KE1, C_KE2, C_VF0, C_VF1, C_VF2, C_VE0, C_VE1, C_VE2, C_SA, C_SB, C_PA, C_PB, C_PA2, C_PB2, C_OA, C_OB, C_DRAIN, C_COUNT };
 
@@ -1070,8 +1071,11 @@ static int sm100_stack_factor(const fa_fwd_params& p) {
     const int G = p.hq / p.hkv;
     return (!p.cu_seqlens_q && p.d <= 128 && p.sq < 128 && G > 1 && G <= 128 && (G & (G - 1)) == 0) ? G : 1;
 }
-// Capped scores without alibi go to the kernel with one query tile a CTA (fwd_single_sm100.cu: the measurements behind
-// this line); alibi, with or without a cap, stays with the BIAS instantiation here.
+// Capped scores without alibi go to the kernel with one query tile a CTA (fwd_single_sm100.cu); alibi, with or without a cap,
+// stays with the BIAS instantiation here.  Two-tile against one-tile kernel, us: inside the range of the tanh polynomial D128
+// B2 S4096 H16 full 1304 / 349, D64 B4 S2048 H16 full 650 / 152, D64 B1 S8192 H16 causal 1195 / 300; beyond it (scores of 8
+// against a cap of 1) D128 B2 S4096 H16 causal 655 / 322, D64 623 / 248; B256 S128 H16 D64 402 / 127; cache calls of four
+// new tokens, B16 up to 32768 keys, 1756 / 419.
 static bool single_tile(const fa_fwd_params& p, int gq, int nsplit) {
     const long blocks = ((long)p.sq * gq + 127) / 128 * nsplit;
     return p.d <= 128 && p.softcap > 0.f && !p.alibi_slopes && blocks <= 65535;        // a grid dimension
