@@ -323,9 +323,9 @@ def workspace_fits(nbytes, device):
     too, beside the 150 or more that kernels with such a workspace run."""
     if nbytes < _LARGE_WORKSPACE or torch.cuda.is_current_stream_capturing():
         return True
-    stats = torch.cuda.memory.memory_stats_as_nested_dict(device)
     try:
+        stats = torch.cuda.memory.memory_stats_as_nested_dict(device)
         held = stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"]
-    except KeyError:                                         # an allocator that keeps no such counts
+    except (KeyError, RuntimeError):                         # an allocator that keeps no such counts
         return True
     return nbytes <= held or nbytes <= held + torch.cuda.mem_get_info(device)[0]

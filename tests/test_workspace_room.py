@@ -25,6 +25,15 @@ def test_what_fits(nbytes, held, free, fits, asked, monkeypatch):
     assert capi.workspace_fits(nbytes, 0)
 
 
+def test_an_allocator_without_counts_is_simply_asked(monkeypatch):
+    """A pluggable allocator refuses the question with a RuntimeError."""
+    def refuse(device=None):
+        raise RuntimeError("not supported")
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(torch.cuda.memory, "memory_stats_as_nested_dict", refuse)
+    assert capi.workspace_fits(3 * GIB, 0)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("d,kernel", [(128, "sm100_tcgen05_bwd"), (256, "generic_mma_bwd")])
 def test_backward_does_not_try_what_cannot_fit(d, kernel, monkeypatch):
