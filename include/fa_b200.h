@@ -162,8 +162,9 @@ typedef struct {
 int    fa_bwd(const fa_bwd_params* p);
 int    fa_varlen_bwd(const fa_bwd_params* p);
 size_t fa_bwd_workspace_bytes(const fa_bwd_params* p);
-/* The least workspace the backward runs with.  Between this and fa_bwd_workspace_bytes() it recomputes for dQ what it would
- * have stored (head dims up to 128) or takes the general kernels, which store nothing (above). */
+/* The least workspace the backward runs with.  Between this and fa_bwd_workspace_bytes(), or on an address that is not 16-byte
+ * aligned, it recomputes for dQ what it would have stored (head dims up to 128) or takes the general kernels, which store
+ * nothing (above). */
 size_t fa_bwd_workspace_min_bytes(const fa_bwd_params* p);
 
 /* ------------------------------------------------------------------------
